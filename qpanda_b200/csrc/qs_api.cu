@@ -303,10 +303,13 @@ void qs_lowstage_passes(const std::vector<qs_prim> &prims, int n, int dtype, boo
                         std::vector<qs_low::Pass> &out);
 int qs_launch_lowstage(qs_state *s, const std::vector<qs_prim> &run, uint64_t qmask);
 
-// Gate by gate, except that runs of consecutive gates whose targets lie
-// within one tile's 10 qubits go through shared memory and registers in one
-// pass each (qs_lowstage.cu) when that moves fewer bytes than the gates would
-// one by one: same arithmetic per amplitude, fewer passes over HBM.
+// qs_stage.cu
+int qs_stage_min_qubits();
+int qs_stage_apply(qs_state *s, const std::vector<qs_prim> &prims);
+
+// Many gates per read and write of the state: staged passes (qs_stage.cu) on
+// states of qs_stage_min_qubits() qubits and more; on narrower ones, runs of
+// consecutive gates through k_lowstage (qs_lowstage.cu).
 extern "C" int qs_gates_apply(qs_state *s, const qs_gate *g, size_t count)
 {
     int r = qs_check_state(s);
@@ -315,6 +318,8 @@ extern "C" int qs_gates_apply(qs_state *s, const qs_gate *g, size_t count)
     std::vector<qs_prim> prims(count);
     for (size_t i = 0; i < count; ++i)
         if ((r = qs_lower_gate(s->n, &g[i], &prims[i]))) return r;
+    if (count == 1) return qs_launch_prim(s, prims[0]);
+    if (s->n >= qs_stage_min_qubits()) return qs_stage_apply(s, prims);
     std::vector<qs_low::Pass> passes;
     qs_lowstage_passes(prims, s->n, s->dtype, false, passes);
     std::vector<qs_prim> run;

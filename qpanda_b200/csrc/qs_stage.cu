@@ -1,0 +1,224 @@
+// qs_stage.cu - the kernel of the staged passes (plan and arithmetic: qs_stage.h).
+#include <atomic>
+#include <vector>
+
+#include "qs_common.cuh"
+#include "qs_stage.h"
+
+namespace {
+
+using namespace qs_stg;
+
+template <typename T, typename R>
+__global__ void __launch_bounds__(1 << (kMaxTile - Traits<T>::RB), sizeof(T) == 4 ? 4 : 2)
+k_stage(T *__restrict__ a, const __grid_constant__ R P)
+{
+    constexpr int RB = Traits<T>::RB, NR = 1 << RB;
+    typedef typename vec2<T>::type V;
+    extern __shared__ __align__(16) unsigned char stage_smem[];
+    V *tile = reinterpret_cast<V *>(stage_smem);
+    V *pa = reinterpret_cast<V *>(a);
+    const uint32_t t = threadIdx.x;
+    const uint64_t base = tile_base(P, blockIdx.x);
+    Regs<T, RB> v;
+    {
+        uint64_t off = base;
+#pragma unroll
+        for (int j = 0; j < kMaxThreadBits; ++j) off |= (t >> j & 1) ? P.gin_t[j] : 0ull;
+        const V *p = pa + off;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            uint64_t ro = 0;
+#pragma unroll
+            for (int j = 0; j < RB; ++j) ro += (r >> j & 1) ? P.gin_r[j] : 0ull;
+            const V x = p[ro];
+            v.r[r] = x.x;
+            v.i[r] = x.y;
+        }
+    }
+    // the ladders' factors, while the loads are in flight
+    V *lane_f = tile + (1u << P.K), *warp_f = lane_f + 32 * P.nladders;
+    if (P.nladders) {
+        const uint32_t lw = P.K - RB - 5;                      // log2 of the CTA's warps
+        for (uint32_t i = t; i < 32u * P.nladders; i += blockDim.x) {
+            double fr, fi;
+            ladder_lane(P, i >> 5, i & 31, fr, fi);
+            lane_f[i] = V{(T)fr, (T)fi};
+        }
+        for (uint32_t i = t; i < (uint32_t)P.nladders << lw; i += blockDim.x) {
+            double fr, fi;
+            ladder_warp(P, i >> lw, i & ((1u << lw) - 1), base, fr, fi);
+            warp_f[i] = V{(T)fr, (T)fi};
+        }
+        __syncthreads();
+    }
+    uint32_t slot = 0;
+    for (int s = 0; s < P.nstages; ++s) {
+        const Stage &st = P.st[s];
+        uint32_t tt = 0;
+#pragma unroll
+        for (int j = 0; j < kMaxThreadBits; ++j) tt ^= (t >> j & 1) ? st.tb[j] : 0u;
+        if (s) {
+            // to the new stage's registers through shared memory.  The slots
+            // written are the ones this thread read at the stage before, so
+            // one barrier is enough.
+            const Stage &sp = P.st[s - 1];
+            uint32_t pr[4];
+#pragma unroll
+            for (int j = 0; j < RB; ++j) pr[j] = sp.pr[j];
+#pragma unroll
+            for (int r = 0; r < NR; ++r) tile[slot ^ reg_xor<RB>(r, pr)] = V{v.r[r], v.i[r]};
+            __syncthreads();
+            slot = tt >> 16;
+#pragma unroll
+            for (int j = 0; j < RB; ++j) pr[j] = st.pr[j];
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const V x = tile[slot ^ reg_xor<RB>(r, pr)];
+                v.r[r] = x.x;
+                v.i[r] = x.y;
+            }
+        }
+        slot = tt >> 16;
+        const uint32_t ti = tt & 0xffffu;
+        const int end = st.first + st.count;
+        for (int o = st.first; o < end; ++o) {
+            const Op<T> &op = P.op[o];
+            if ((base & op.need) != op.need) continue;         // the same for the whole CTA
+            if ((ti & op.cthr) != op.cthr) continue;
+            T fr = 1, fi = 0;
+            if (op.kind >= K_LADR && op.kind <= K_LAD0) {
+                const uint32_t lw = P.K - RB - 5;
+                const V x = lane_f[32 * op.ladder + (t & 31)], y = warp_f[(op.ladder << lw) + (t >> 5)];
+                fr = x.x;
+                fi = x.y;
+                cmul(fr, fi, y.x, y.y);
+            }
+            apply_op<T, RB>(v, op, fr, fi);
+        }
+    }
+    {
+        uint64_t off = base;
+#pragma unroll
+        for (int j = 0; j < kMaxThreadBits; ++j) off |= (t >> j & 1) ? P.gout_t[j] : 0ull;
+        if (P.scale_kind == 1) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) { v.r[r] *= P.scale[0]; v.i[r] *= P.scale[0]; }
+        } else if (P.scale_kind == 2) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) cmul(v.r[r], v.i[r], P.scale[0], P.scale[1]);
+        }
+        V *p = pa + off;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            uint64_t ro = 0;
+#pragma unroll
+            for (int j = 0; j < RB; ++j) ro += (r >> j & 1) ? P.gout_r[j] : 0ull;
+            p[ro] = V{v.r[r], v.i[r]};
+        }
+    }
+}
+
+template <typename T, typename R>
+int launch(qs_state *s, const R &P)
+{
+    const size_t amps = (1ull << P.K) + (size_t)P.nladders * (32 + (1u << (P.K - Traits<T>::RB - 5)));
+    const size_t smem = 2 * sizeof(T) * amps;
+    if (smem > 48 * 1024) {
+        // once per device and kernel: the largest a pass can need
+        static std::atomic<uint64_t> done{0};
+        const uint64_t bit = 1ull << (s->device & 63);
+        if (!(done.load() & bit)) {
+            const int most = (int)(2 * sizeof(T) * ((1u << kMaxTile) + R::NLAD * (32 + (1u << (kMaxTile - Traits<T>::RB - 5)))));
+            QS_CUDA_TRY(cudaFuncSetAttribute(k_stage<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+            done.fetch_or(bit);
+        }
+    }
+    k_stage<T, R><<<(unsigned)(s->N >> P.K), 1u << (P.K - Traits<T>::RB), smem, s->stream>>>(static_cast<T *>(s->amp), P);
+    QS_LAUNCH_CHECK("k_stage");
+    return QS_OK;
+}
+
+// one op on the per-gate kernels
+int launch_op(qs_state *s, const Planner &P, const GOp &g)
+{
+    int r = QS_OK;
+    if (g.type == G_U || (g.type == G_DIAG && g.ctrl == 0)) {
+        const uint64_t t = g.type == G_U ? g.tgt : g.off1;
+        return launch_pair(s, t, 0, 0, t, g.m);
+    }
+    if (g.type == G_DIAG) {
+        for (int k = g.first; !r && k < g.first + g.count; ++k) {
+            const Term &t = P.terms[(size_t)k];
+            r = launch_phase(s, g.ctrl | (t.q >= 0 ? 1ull << t.q : 0), t.re, t.im);
+        }
+        return r;
+    }
+    if (g.type == G_CU) return launch_pair(s, g.tgt | g.ctrl, g.ctrl, 0, g.tgt, g.m);
+    return launch_pair(s, g.tgt | g.ctrl, g.ctrl, g.off0, g.off1, g.m);
+}
+
+// HBM traffic of an op on the per-gate kernels, in passes over the state,
+// in whole 32-byte sectors: each control or phase bit above the sector halves
+// it, and so does an exchange whose higher bit is.
+double op_traffic(const Planner &P, const GOp &g)
+{
+    const int sb = P.dtype == QS_C64 ? 2 : 1;
+    auto part = [&](uint64_t bits) { return std::ldexp(1.0, -__builtin_popcountll(bits >> sb)); };
+    if (g.type == G_U || (g.type == G_DIAG && g.ctrl == 0)) return 1.0;
+    if (g.type == G_DIAG) {
+        double sum = 0;
+        for (int k = g.first; k < g.first + g.count; ++k) {
+            const Term &t = P.terms[(size_t)k];
+            sum += part(g.ctrl | (t.q >= 0 ? 1ull << t.q : 0));
+        }
+        return sum;
+    }
+    const double c = part(g.ctrl);
+    return g.type == G_CU || !((g.off0 | g.off1) >> sb) ? c : c / 2;
+}
+
+template <typename T>
+int apply_t(qs_state *s, const std::vector<qs_prim> &prims)
+{
+    Planner P(prims, s->n, s->dtype);
+    uint64_t qmask;
+    std::vector<int> pass, rest;
+    RunSmall<T> small;
+    static thread_local RunLarge<T> large;
+    while (P.next(&qmask, &pass)) {
+        // a pass that would move more than its gates one by one stays with them
+        double traffic = 0;
+        for (int i : pass) traffic += op_traffic(P, P.ops[(size_t)i]);
+        int r = QS_OK;
+        if (pass.size() == 1 || (traffic <= 1.0 && s->amp_bytes() >= (64ull << 20))) {
+            for (size_t k = 0; !r && k < pass.size(); ++k) r = launch_op(s, P, P.ops[(size_t)pass[k]]);
+            if (r) return r;
+            continue;
+        }
+        bool done = false;
+        if ((int)pass.size() < RunSmall<T>::NOP - 1) {
+            plan_pass<RunSmall<T>, T>(P, qmask, pass, &small, &rest);
+            done = rest.empty();
+            if (done) r = launch<T>(s, small);
+        }
+        if (!done) {
+            plan_pass<RunLarge<T>, T>(P, qmask, pass, &large, &rest);
+            if (!rest.empty()) P.give_back(rest);
+            r = launch<T>(s, large);
+        }
+        if (r) return r;
+    }
+    return QS_OK;
+}
+
+}  // namespace
+
+// Apply a lowered gate list with staged passes (states of kMinTile qubits and
+// more); asynchronous on the state's stream.
+int qs_stage_apply(qs_state *s, const std::vector<qs_prim> &prims)
+{
+    return s->dtype == QS_C64 ? apply_t<float>(s, prims) : apply_t<double>(s, prims);
+}
+
+int qs_stage_min_qubits() { return kMinTile; }

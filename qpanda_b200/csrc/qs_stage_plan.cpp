@@ -1,0 +1,572 @@
+// qs_stage_plan.cpp - planner of the staged passes (qs_stage.h): gate list ->
+// simplified ops -> passes -> stages.  Host-only.
+#include <algorithm>
+#include <complex>
+
+#include "qs_stage.h"
+
+namespace qs_stg {
+
+namespace {
+
+typedef std::complex<double> cd;
+
+inline int popc(uint64_t x) { return __builtin_popcountll(x); }
+inline int low_bit(uint64_t x) { return __builtin_ctzll(x); }
+
+bool is_x(const double m[8])
+{
+    return m[0] == 0 && m[1] == 0 && m[2] == 1 && m[3] == 0 && m[4] == 1 && m[5] == 0 && m[6] == 0 && m[7] == 0;
+}
+
+bool is_diag(const double m[8]) { return m[2] == 0 && m[3] == 0 && m[4] == 0 && m[5] == 0; }
+
+// a := b * a, 2x2 row-major complex
+void mul2(double a[8], const double b[8])
+{
+    const cd a00(a[0], a[1]), a01(a[2], a[3]), a10(a[4], a[5]), a11(a[6], a[7]);
+    const cd b00(b[0], b[1]), b01(b[2], b[3]), b10(b[4], b[5]), b11(b[6], b[7]);
+    const cd c[4] = {b00 * a00 + b01 * a10, b00 * a01 + b01 * a11, b10 * a00 + b11 * a10, b10 * a01 + b11 * a11};
+    for (int k = 0; k < 4; ++k) {
+        a[2 * k] = c[k].real();
+        a[2 * k + 1] = c[k].imag();
+    }
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------ the simplified gate list
+Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_), dtype(dtype_)
+{
+    K = n < kMaxTile ? n : kMaxTile;
+    low = dtype == QS_C64 ? Traits<float>::LOW : Traits<double>::LOW;
+    ops.reserve(prims.size());
+    int open[64];                          // the 1-qubit op that a gate on this qubit may join
+    for (int &o : open) o = -1;
+    int last_diag = -1;                    // the phase op that another phase may join ...
+    uint64_t since = 0;                    // ... and the qubits mixed after it
+    for (size_t i = 0; i < prims.size(); ++i) {
+        const qs_prim &p = prims[i];
+        if (p.kind == QS_PRIM_PAIR && p.off0 == 0 && p.cmask == 0) {
+            const int q = low_bit(p.off1);
+            if (open[q] >= 0) {
+                mul2(ops[open[q]].m, p.m);
+                ++ops[open[q]].nprims;
+                continue;
+            }
+            GOp g = {};
+            g.type = G_U;
+            g.tgt = p.off1;
+            memcpy(g.m, p.m, sizeof(g.m));
+            g.nprims = 1;
+            open[q] = (int)ops.size();
+            since |= g.tgt;
+            ops.push_back(g);
+            continue;
+        }
+        for (uint64_t h = p.holes; h; h &= h - 1) open[low_bit(h)] = -1;
+        if (p.kind == QS_PRIM_PHASE) {
+            if (last_diag >= 0 && !(since & p.holes)) {
+                // join the last phase op when every term then has at most one
+                // qubit beside a common hub
+                GOp &d = ops[last_diag];
+                const uint64_t hub = d.ctrl & p.holes;
+                const uint64_t mine = p.holes & ~hub, first = d.ctrl & ~hub;
+                if (hub && popc(mine) <= 1 && (first == 0 || (d.count == 1 && popc(first) == 1)) &&
+                    d.first + d.count == (int)terms.size()) {
+                    if (first) terms[d.first].q = low_bit(first);
+                    d.ctrl = hub;
+                    d.diag |= p.holes;
+                    terms.push_back({mine ? low_bit(mine) : -1, p.m[0], p.m[1]});
+                    ++d.count;
+                    ++d.nprims;
+                    continue;
+                }
+            }
+            GOp g = {};
+            g.type = G_DIAG;
+            g.diag = g.ctrl = p.holes;
+            g.m[0] = 1;
+            g.first = (int)terms.size();
+            g.count = 1;
+            g.nprims = 1;
+            terms.push_back({-1, p.m[0], p.m[1]});
+            last_diag = (int)ops.size();
+            since = 0;
+            ops.push_back(g);
+            continue;
+        }
+        GOp g = {};
+        memcpy(g.m, p.m, sizeof(g.m));
+        g.nprims = 1;
+        g.ctrl = g.diag = p.cmask;
+        if (p.off0 == 0) {
+            g.type = G_CU;
+            g.tgt = p.off1;
+        } else {
+            g.type = p.cmask == 0 && is_x(p.m) ? G_SWAP : G_EX;
+            g.tgt = p.off0 | p.off1;
+            g.off0 = p.off0;
+            g.off1 = p.off1;
+        }
+        since |= g.tgt;
+        ops.push_back(g);
+    }
+    // diagonal 1-qubit ops mix nothing: a factor m00 of everything (m00 on the
+    // controls' subspace) and a phase m11 / m00 where the qubit is set
+    for (GOp &g : ops) {
+        if ((g.type != G_U && g.type != G_CU) || !is_diag(g.m)) continue;
+        const cd m00(g.m[0], g.m[1]), w = cd(g.m[6], g.m[7]) / m00;
+        g.first = (int)terms.size();
+        g.count = 0;
+        if (g.type == G_CU && !(m00 == cd(1, 0))) {
+            terms.push_back({-1, m00.real(), m00.imag()});
+            ++g.count;
+        }
+        terms.push_back({low_bit(g.tgt), w.real(), w.imag()});
+        ++g.count;
+        g.diag |= g.tgt;
+        g.off1 = g.tgt;
+        g.tgt = 0;
+        g.type = G_DIAG;
+    }
+    left.resize(ops.size());
+    for (size_t i = 0; i < ops.size(); ++i) left[i] = (int)i;
+}
+
+// Ops of `left` that can run in a pass on the tile of q: their targets in q,
+// and they commute with every earlier op that stays behind.  Returns their
+// number; *taken gets them, *wants the target sets that alone keep an op out.
+int Planner::scan(uint64_t q, std::vector<uint64_t> *wants, std::vector<int> *taken) const
+{
+    const uint64_t all = n >= 64 ? ~0ull : (1ull << n) - 1;
+    uint64_t skip_all = 0, skip_tgt = 0;
+    int count = 0;
+    for (int i : left) {
+        const GOp &g = ops[(size_t)i];
+        const bool free = !(g.tgt & skip_all) && !(g.diag & skip_tgt);
+        if (free && !(g.tgt & ~q)) {
+            ++count;
+            if (taken) taken->push_back(i);
+            continue;
+        }
+        if (free && wants) {
+            const uint64_t w = g.tgt & ~q;
+            if (popc(q | w) <= K && std::find(wants->begin(), wants->end(), w) == wants->end()) wants->push_back(w);
+        }
+        skip_all |= g.tgt | g.diag;
+        skip_tgt |= g.tgt;
+        if ((skip_tgt & all) == all) break;
+    }
+    return count;
+}
+
+bool Planner::next(uint64_t *qmask, std::vector<int> *pass_ops)
+{
+    pass_ops->clear();
+    if (left.empty()) return false;
+    uint64_t q = n <= K ? (1ull << n) - 1 : (1ull << low) - 1;
+    if (n > K) {
+        // grow the tile by the target set that lets the most ops per qubit in
+        int have = scan(q, nullptr, nullptr);
+        std::vector<uint64_t> wants;
+        while (popc(q) < K) {
+            wants.clear();
+            scan(q, &wants, nullptr);
+            uint64_t best = 0;
+            double best_gain = -1;
+            int best_count = 0;
+            for (uint64_t w : wants) {
+                const int c = scan(q | w, nullptr, nullptr);
+                const double gain = (double)(c - have) / popc(w);
+                if (gain > best_gain) {
+                    best_gain = gain;
+                    best = w;
+                    best_count = c;
+                }
+            }
+            if (!best) break;
+            q |= best;
+            have = best_count;
+        }
+        for (int b = 0; b < n && popc(q) < K; ++b) q |= 1ull << b;
+    }
+    scan(q, nullptr, pass_ops);
+    // left minus pass_ops (both ascending)
+    size_t k = 0, o = 0;
+    for (size_t i = 0; i < left.size(); ++i) {
+        if (k < pass_ops->size() && left[i] == (*pass_ops)[k]) { ++k; continue; }
+        left[o++] = left[i];
+    }
+    left.resize(o);
+    *qmask = q;
+    return true;
+}
+
+void Planner::give_back(const std::vector<int> &rest)
+{
+    std::vector<int> all;
+    all.reserve(left.size() + rest.size());
+    std::merge(left.begin(), left.end(), rest.begin(), rest.end(), std::back_inserter(all));
+    left.swap(all);
+}
+
+// ------------------------------------------------------------------ stages of a pass
+namespace {
+
+// p * [[.., ..], [.., ..]] with the pivot p pulled out: the kind (base + 0),
+// r, q and the factor that is left.  Kinds of dense ops keep the matrix.
+template <typename T>
+uint8_t classify(const double m[8], T *out, double *p)
+{
+    *p = 1;
+    for (int k = 0; k < 8; ++k) out[k] = (T)m[k];
+    if (is_x(m)) return K_X;
+    const double tol = 9e-16;            // 4 ulp: products of a few rotations
+    double r, q, piv;
+    uint8_t kind = K_GEN;
+    if (m[1] == 0 && m[3] == 0 && m[5] == 0 && m[7] == 0) {
+        if (std::fabs(m[0]) >= std::fabs(m[2])) {
+            piv = m[0]; r = m[2] / piv; q = m[4] / piv;
+            if (std::fabs(m[6] / piv - 1) < tol) kind = K_RAP;
+            else if (std::fabs(m[6] / piv + 1) < tol) kind = K_RAM;
+        } else {
+            piv = m[2]; r = m[0] / piv; q = m[6] / piv;
+            if (std::fabs(m[4] / piv - 1) < tol) kind = K_RBP;
+            else if (std::fabs(m[4] / piv + 1) < tol) kind = K_RBM;
+        }
+    } else if (m[1] == 0 && m[7] == 0 && m[2] == 0 && m[4] == 0) {
+        if (std::fabs(m[0]) >= std::fabs(m[3])) {
+            piv = m[0]; r = m[3] / piv; q = m[5] / piv;
+            if (std::fabs(m[6] / piv - 1) < tol) kind = K_IA;
+        } else {
+            piv = m[3]; r = m[0] / piv; q = m[6] / piv;
+            if (std::fabs(m[5] / piv - 1) < tol) kind = K_IB;
+        }
+    }
+    if (kind == K_GEN) return kind;
+    out[0] = (T)r;
+    out[1] = (T)q;
+    *p = piv;
+    // r and q rounded to T turn the angle by that rounding; the factor follows,
+    // so that the gate stays unitary to FP64 rounding
+    if (std::fabs(r) == std::fabs(q)) {
+        const double rt = (double)out[0];
+        *p *= std::sqrt((1 + r * r) / (1 + rt * rt));
+    }
+    return kind;
+}
+
+int pair_index(int ja, int jb) { return jb * (jb - 1) / 2 + ja; }
+
+}  // namespace
+
+template <typename R, typename T>
+void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_ops, R *out, std::vector<int> *rest)
+{
+    constexpr int RB = Traits<T>::RB, LB = Traits<T>::LB, LOW = Traits<T>::LOW;
+    const int K = popc(qmask), n = P.n, tbits = K - RB;
+    R &S = *out;
+    S.K = K;
+    S.nstages = S.nladders = 0;
+    S.pad = 0;
+    memset(S.gin_t, 0, sizeof(S.gin_t));
+    memset(S.gin_r, 0, sizeof(S.gin_r));
+    memset(S.gout_t, 0, sizeof(S.gout_t));
+    memset(S.gout_r, 0, sizeof(S.gout_r));
+    rest->clear();
+    // tile bit of a qubit, and the qubit of a tile bit at the load
+    int pos[64], qubit[kMaxTile];
+    {
+        int k = 0;
+        for (int q = 0; q < n; ++q) {
+            pos[q] = -1;
+            if (qmask >> q & 1) {
+                qubit[k] = q;
+                pos[q] = k++;
+            }
+        }
+    }
+    // the tile index's bits go to the qubits outside the tile, run by run
+    S.nseg = 0;
+    for (int q = 0, from = 0; q < n;) {
+        if (qmask >> q & 1) { ++q; continue; }
+        int len = 0;
+        while (q + len < n && !(qmask >> (q + len) & 1)) ++len;
+        S.seg_mask[S.nseg] = ((1ull << len) - 1) << from;
+        S.seg_shift[S.nseg] = (uint8_t)(q - from);
+        ++S.nseg;
+        from += len;
+        q += len;
+    }
+    auto tile_bits = [&](uint64_t qs, const int *ps) {
+        uint32_t o = 0;
+        for (qs &= qmask; qs; qs &= qs - 1) o |= 1u << ps[low_bit(qs)];
+        return o;
+    };
+    std::vector<int> todo(pass_ops), take;
+    // ops of todo that run in a stage with these register bits (tile bits)
+    auto scan = [&](uint32_t regs, std::vector<uint32_t> *wants, std::vector<int> *taken) {
+        uint64_t skip_all = 0, skip_tgt = 0;
+        int count = 0, ps[64];
+        bool moved = false;
+        const int *cur = pos;
+        for (int i : todo) {
+            const GOp &g = P.ops[(size_t)i];
+            const bool free = !(g.tgt & skip_all) && !(g.diag & skip_tgt);
+            if (free) {
+                if (g.type == G_SWAP) {
+                    if (!moved) {
+                        memcpy(ps, pos, sizeof(ps));
+                        cur = ps;
+                        moved = true;
+                    }
+                    std::swap(ps[low_bit(g.off0)], ps[low_bit(g.off1)]);
+                    if (taken) taken->push_back(i);
+                    continue;
+                }
+                const uint32_t t = tile_bits(g.tgt, cur);
+                if (!(t & ~regs)) {
+                    count += g.tgt ? 2 : 0;        // what needs no register bit runs in any stage
+                    if (taken) taken->push_back(i);
+                    continue;
+                }
+                const uint32_t w = t & ~regs;
+                if (wants && popc(regs | w) <= RB && std::find(wants->begin(), wants->end(), w) == wants->end())
+                    wants->push_back(w);
+            }
+            skip_all |= g.tgt | g.diag;
+            skip_tgt |= g.tgt;
+            if ((skip_tgt & qmask) == qmask) break;
+        }
+        return count;
+    };
+    cd scale(1, 0);
+    double growth = 1;
+    int nops = 0, nent = 0;
+    const uint32_t low_tile = (1u << LOW) - 1, all_tile = (1u << K) - 1;
+    auto choose = [&](uint32_t allowed) {
+        uint32_t regs = 0;
+        std::vector<uint32_t> wants;
+        int have = scan(0, nullptr, nullptr);
+        while (popc(regs) < RB) {
+            wants.clear();
+            scan(regs, &wants, nullptr);
+            uint32_t best = 0;
+            double best_gain = -1;
+            int best_count = 0;
+            for (uint32_t w : wants) {
+                if (w & ~allowed) continue;
+                const int c = scan(regs | w, nullptr, nullptr);
+                const double gain = (double)(c - have) / popc(w);
+                if (gain > best_gain) { best_gain = gain; best = w; best_count = c; }
+            }
+            if (!best) break;
+            regs |= best;
+            have = best_count;
+        }
+        for (int b = K - 1; b >= 0 && popc(regs) < RB; --b)
+            if (allowed >> b & 1) regs |= 1u << b;
+        return regs;
+    };
+    // the stage's layout; lanes: the tile bits that must come first, in order
+    int thread_of[kMaxTile], reg_of[kMaxTile];
+    auto add_stage = [&](uint32_t regs, const int *lanes, int nlanes) {
+        Stage &st = S.st[S.nstages++];
+        memset(&st, 0, sizeof(st));
+        st.first = (uint16_t)nops;
+        int order[kMaxTile], no = 0;
+        uint32_t basis[4] = {0, 0, 0, 0}, used = regs;
+        auto independent = [&](int b) {
+            uint32_t v = bit_image<T>(b);
+            for (int h = LB - 1; h >= 0; --h)
+                if ((v >> h & 1) && basis[h]) v ^= basis[h];
+            if (!v) return false;
+            basis[31 - __builtin_clz(v)] = v;
+            return true;
+        };
+        for (int j = 0; j < nlanes; ++j) {
+            order[no++] = lanes[j];
+            used |= 1u << lanes[j];
+            independent(lanes[j]);
+        }
+        for (int b = 0; b < K && no < LB; ++b)
+            if (!(used >> b & 1) && independent(b)) {
+                order[no++] = b;
+                used |= 1u << b;
+            }
+        for (int b = 0; b < K; ++b)
+            if (!(used >> b & 1)) order[no++] = b;
+        for (int b = 0; b < K; ++b) thread_of[b] = reg_of[b] = -1;
+        for (int j = 0; j < tbits; ++j) {
+            st.tb[j] = (1u << order[j]) | bit_slot<T>(order[j]) << 16;
+            thread_of[order[j]] = j;
+        }
+        int j = 0;
+        for (int b = 0; b < K; ++b)
+            if (regs >> b & 1) {
+                st.pr[j] = (uint16_t)bit_slot<T>(b);
+                reg_of[b] = j++;
+            }
+        return &st;
+    };
+    const uint64_t outside = ~qmask;
+    // masks of a condition on qubits, by where each lies now
+    auto condition = [&](uint64_t qs, Op<T> *op) {
+        op->need = qs & outside;
+        op->cthr = 0;
+        op->creg = 0;
+        const uint32_t tb = tile_bits(qs, pos);
+        for (int b = 0; b < K; ++b)
+            if (tb >> b & 1) {
+                if (reg_of[b] >= 0) op->creg |= 1u << reg_of[b];
+                else op->cthr |= 1u << b;
+            }
+    };
+    auto reg_bit = [&](uint64_t qs) { return reg_of[pos[low_bit(qs)]]; };
+    // one op at the current stage; false when it does not fit the parameter block
+    auto emit = [&](const GOp &g) {
+        if (g.type == G_SWAP) {
+            std::swap(pos[low_bit(g.off0)], pos[low_bit(g.off1)]);
+            return true;
+        }
+        if (nops + 2 > R::NOP) return false;
+        Op<T> &op = S.op[nops];
+        memset(&op, 0, sizeof(op));
+        if (g.type == G_U) {
+            double p;
+            op.kind = (uint8_t)(classify<T>(g.m, op.m, &p) + reg_bit(g.tgt));
+            scale *= p;
+            growth /= std::fabs(p);
+        } else if (g.type == G_CU) {
+            condition(g.ctrl, &op);
+            for (int k = 0; k < 8; ++k) op.m[k] = (T)g.m[k];
+            const bool x = is_x(g.m);
+            op.kind = (uint8_t)((x ? (op.creg ? K_XR : K_X) : (op.creg ? K_GENR : K_GEN)) + reg_bit(g.tgt));
+        } else if (g.type == G_EX) {
+            condition(g.ctrl, &op);
+            int ja = reg_bit(g.off0), jb = reg_bit(g.off1);
+            for (int k = 0; k < 8; ++k) op.m[k] = (T)(ja < jb ? g.m[k] : g.m[6 - 2 * (k / 2) + (k & 1)]);
+            if (ja > jb) std::swap(ja, jb);
+            op.kind = (uint8_t)(K_EX + pair_index(ja, jb));
+        } else if (g.count == 1) {
+            const Term &t = P.terms[(size_t)g.first];
+            condition(g.ctrl | (t.q >= 0 ? 1ull << t.q : 0), &op);
+            op.m[0] = (T)t.re;
+            op.m[1] = (T)t.im;
+            op.kind = op.creg == 0 ? K_PH0 : (op.creg & (op.creg - 1)) ? K_PHR : K_PH + low_bit(op.creg);
+        } else {
+            if (S.nladders == R::NLAD || nent + g.count > R::NENT) return false;
+            condition(g.ctrl, &op);
+            for (int j = 0; j < RB; ++j) op.m[2 * j] = 1;
+            op.ladder = (uint32_t)S.nladders;
+            Ladder &L = S.lad[S.nladders++];
+            L.first = (uint16_t)nent;
+            L.nthr = L.nout = L.pad = 0;
+            for (int side = 0; side < 2; ++side)
+                for (int k = 0; k < g.count; ++k) {
+                    const Term &t = P.terms[(size_t)(g.first + k)];
+                    // a term on the hub alone: any of the hub's qubits carries it
+                    const int q = t.q >= 0 ? t.q : low_bit(g.ctrl);
+                    const bool out_q = outside >> q & 1;
+                    if (!out_q && reg_of[pos[q]] >= 0) {
+                        if (side) continue;
+                        T *w = &op.m[2 * reg_of[pos[q]]];
+                        const cd z = cd(t.re, t.im) * cd((double)w[0], (double)w[1]);
+                        w[0] = (T)z.real();
+                        w[1] = (T)z.imag();
+                    } else if (out_q == (side == 1)) {
+                        S.ent[nent++] = {t.re, t.im, out_q ? q : thread_of[pos[q]], 0};
+                        ++(out_q ? L.nout : L.nthr);
+                    }
+                }
+            op.kind = op.creg == 0 ? K_LAD0 : (op.creg & (op.creg - 1)) ? K_LADR : K_LAD + low_bit(op.creg);
+        }
+        if (g.type == G_DIAG && g.ctrl == 0) scale *= cd(g.m[0], g.m[1]);
+        ++nops;
+        if (growth > 0x1p8) {                     // the pivots' factors so far, before values grow further
+            Op<T> &sc = S.op[nops++];
+            memset(&sc, 0, sizeof(sc));
+            const double s = std::abs(scale);
+            sc.kind = K_SCALE;
+            sc.m[0] = (T)s;
+            scale /= (double)sc.m[0];
+            growth = 1;
+        }
+        return true;
+    };
+    bool full = false, stored = false;
+    while (!stored) {
+        const bool first = S.nstages == 0;
+        const uint32_t regs = choose(first ? all_tile & ~low_tile : all_tile);
+        take.clear();
+        scan(regs, nullptr, &take);
+        // the store reads the tile with the lowest qubits on the lowest lanes
+        int ps[64], lanes[LOW];
+        memcpy(ps, pos, sizeof(ps));
+        for (int i : take) {
+            const GOp &g = P.ops[(size_t)i];
+            if (g.type == G_SWAP) std::swap(ps[low_bit(g.off0)], ps[low_bit(g.off1)]);
+        }
+        bool last = take.size() == todo.size();
+        for (int q = 0; q < LOW; ++q) {
+            lanes[q] = ps[q];
+            last = last && !(regs >> ps[q] & 1);
+        }
+        static const int natural[4] = {0, 1, 2, 3};
+        // one stage alone has no barrier between its loads and its stores:
+        // every thread must then store where it loaded
+        if (first && last) last = memcmp(ps, pos, sizeof(int) * (size_t)n) == 0;
+        Stage *st = add_stage(regs, first ? natural : lanes, first || last ? LOW : 0);
+        size_t k = 0, t = 0;
+        for (; k < take.size(); ++k)
+            if (!emit(P.ops[(size_t)take[k]])) {
+                full = true;
+                break;
+            }
+        st->count = (uint16_t)(nops - st->first);
+        // todo minus what was emitted
+        for (size_t i = 0, e = 0; i < todo.size(); ++i) {
+            if (e < k && todo[i] == take[e]) { ++e; continue; }
+            todo[t++] = todo[i];
+        }
+        todo.resize(t);
+        if (full || S.nstages + 1 >= R::NST) {
+            *rest = todo;
+            todo.clear();
+            full = true;
+        }
+        stored = last && !full;
+        if (stored || todo.empty()) {
+            if (!stored) {
+                for (int q = 0; q < LOW; ++q) lanes[q] = pos[q];
+                uint32_t low_now = 0, regs2 = 0;
+                for (int q = 0; q < LOW; ++q) low_now |= 1u << lanes[q];
+                for (int b = K - 1; b >= 0 && popc(regs2) < RB; --b)
+                    if (!(low_now >> b & 1)) regs2 |= 1u << b;
+                add_stage(regs2, lanes, LOW)->count = 0;
+                stored = true;
+            }
+        }
+    }
+    // state offsets of the load (first stage) and the store (last stage)
+    int at[kMaxTile];                              // qubit behind a tile bit at the store
+    for (int q = 0; q < n; ++q)
+        if (pos[q] >= 0) at[pos[q]] = q;
+    auto offsets = [&](const Stage &st, const int *qs, uint64_t *gt, uint64_t *gr) {
+        for (int j = 0; j < tbits; ++j) gt[j] = 1ull << qs[low_bit(st.tb[j] & 0xffffu)];
+        for (int j = 0; j < RB; ++j) gr[j] = 1ull << qs[31 - __builtin_clz((uint32_t)st.pr[j])];
+    };
+    offsets(S.st[0], qubit, S.gin_t, S.gin_r);
+    offsets(S.st[S.nstages - 1], at, S.gout_t, S.gout_r);
+    S.scale[0] = (T)scale.real();
+    S.scale[1] = (T)scale.imag();
+    S.scale_kind = scale.imag() != 0 ? 2 : scale.real() != 1 ? 1 : 0;
+}
+
+template void plan_pass<RunSmall<float>, float>(const Planner &, uint64_t, const std::vector<int> &, RunSmall<float> *, std::vector<int> *);
+template void plan_pass<RunLarge<float>, float>(const Planner &, uint64_t, const std::vector<int> &, RunLarge<float> *, std::vector<int> *);
+template void plan_pass<RunSmall<double>, double>(const Planner &, uint64_t, const std::vector<int> &, RunSmall<double> *, std::vector<int> *);
+template void plan_pass<RunLarge<double>, double>(const Planner &, uint64_t, const std::vector<int> &, RunLarge<double> *, std::vector<int> *);
+
+}  // namespace qs_stg

@@ -1,0 +1,103 @@
+"""CPU check of the staged passes (no GPU): tests/stage_emu/stage_emu.cpp runs
+gate lists through the library's own planner and the kernel's own per-thread
+functions.  The state must match the oracle to the rounding of its precision,
+every amplitude must be loaded and stored exactly once per pass, every
+shared-memory slot written and read exactly once per stage change, and passes
+without renamed qubits must be free of bank conflicts.
+"""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from oracle.pyoracle import OracleState
+from qpanda_b200 import circuits
+from qpanda_b200.capi import lib
+from tests.golden.make_golden import every_gate_circuit
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+LIBDIR = os.path.join(ROOT, "qpanda_b200", "_lib")
+C64, C128 = 0, 1
+# FP32: a few roundings of 6e-8 per gate on amplitudes below 1, ~150 gates
+TOL = {C64: 1e-6, C128: 1e-14}
+
+
+@pytest.fixture(scope="module")
+def emu(tmp_path_factory):
+    lib()                                     # the library must be built
+    out = str(tmp_path_factory.mktemp("stage_emu") / "libstage_emu.so")
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", os.path.join(ROOT, "tests", "stage_emu", "stage_emu.cpp"),
+           "-I" + os.path.join(ROOT, "qpanda_b200", "csrc"), "-I" + os.path.join(ROOT, "include"), "-L" + LIBDIR,
+           "-lqsb200", "-Wl,-rpath=" + LIBDIR, "-o", out]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    E = C.CDLL(out)
+    E.stage_emu_error.restype = C.c_char_p
+    return E
+
+
+def plan(E, n, gates, dtype, state=None):
+    """Run (or with state=None only plan) the list; (passes, stages, conflicts, ops, small)."""
+    g = np.ascontiguousarray(gates)
+    st = (C.c_longlong * 5)()
+    r = E.stage_emu_apply(None if state is None else state.ctypes.data_as(C.c_void_p), n,
+                          g.ctypes.data_as(C.c_void_p), len(g), dtype, st)
+    assert r == 0, E.stage_emu_error().decode()
+    return list(st)
+
+
+def phases_and_swaps(n, seed):
+    """Ladders on shared hubs, repeated and multi-controlled phases, swaps and
+    controlled gates whose controls and targets lie anywhere."""
+    rng = np.random.default_rng(seed)
+    spec = []
+    for _ in range(60):
+        a, b, c = (int(x) for x in rng.permutation(n)[:3])
+        spec += [("CR", (a, b), 0.3), ("CR", (a, c), -0.7), ("CR", (b, a), 1.1), ("H", (c,)), ("SWAP", (b, c)),
+                 ("RZ", (a,), 0.4), ("CNOT", (c, a)), ("RX", (b,), 2.5), ("RY", (b,), 2.9), ("X", (c,))]
+    g = circuits.make_gates(spec)
+    for k in range(0, len(g), 7):             # QRunes CONTROL lists on every kind of gate
+        free = [q for q in range(n) if q not in g["q"][k][:2]]
+        g["nctrl"][k] = 2
+        g["ctrl"][k][:2] = rng.permutation(free)[:2]
+    return g
+
+
+LISTS = {
+    "layers": lambda n: circuits.random_layers(n, 5, n, iswap_frac=0.3),
+    "qft": circuits.qft,
+    "every": lambda n: every_gate_circuit(n, 11 + n),
+    "ansatz": lambda n: circuits.vqe_ansatz(n, 3, n),
+    "phases": lambda n: phases_and_swaps(n, n),
+    "long": lambda n: circuits.random_layers(n, 40, n),         # several parameter blocks' worth
+}
+
+
+@pytest.mark.parametrize("dtype", [C64, C128])
+@pytest.mark.parametrize("n", [9, 10, 12, 13, 15])
+@pytest.mark.parametrize("kind", list(LISTS))
+def test_passes_match_oracle(emu, kind, n, dtype):
+    rng = np.random.default_rng(7 * n + dtype)
+    init = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    init /= np.linalg.norm(init)
+    gates = LISTS[kind](n)
+    st = init.copy()
+    passes, stages, conflicts, ops, small = plan(emu, n, gates, dtype, st)
+    o = OracleState(n)
+    o.set_state(init)
+    o.apply(gates)
+    assert np.abs(st - o.state()).max() < TOL[dtype] * (4 if kind == "long" else 1)
+    if n >= 12 and kind in ("layers", "ansatz"):
+        assert conflicts == 0
+
+
+@pytest.mark.parametrize("n,gates,dtype,most", [
+    (20, lambda: circuits.random_layers(20, 20, 20240601), C128, 14),
+    (32, lambda: circuits.random_layers(32, 16, 20240601, iswap_frac=0.1), C64, 24),
+    (28, lambda: circuits.qft(28), C64, 6),
+    (28, lambda: circuits.qft(28), C128, 6),
+])
+def test_benchmark_circuits_run_in_few_passes(emu, n, gates, dtype, most):
+    assert plan(emu, n, gates(), dtype)[0] <= most
