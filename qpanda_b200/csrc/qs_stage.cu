@@ -18,28 +18,32 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
     extern __shared__ __align__(16) unsigned char stage_smem[];
     V *tile = reinterpret_cast<V *>(stage_smem);
     V *pa = reinterpret_cast<V *>(a);
+    constexpr int LOW = Traits<T>::LOW;
     const uint32_t t = threadIdx.x;
     const uint64_t base = tile_base(P, blockIdx.x);
     Regs<T, RB> v;
-    {
-        uint64_t off = base;
+    // the state address of a thread's register r: thread part + register part
+    // (the same for all threads), both in units of 2^LOW amplitudes
+    auto thread_at = [&](const uint32_t *gt) {
+        uint32_t u = 0;
 #pragma unroll
-        for (int j = 0; j < kMaxThreadBits; ++j) off |= (t >> j & 1) ? P.gin_t[j] : 0ull;
-        const V *p = pa + off;
+        for (int j = LOW; j < kMaxThreadBits; ++j) u += (t >> j & 1) * gt[j];
+        return pa + base + (t & ((1u << LOW) - 1)) + ((uint64_t)u << LOW);
+    };
+    auto reg_at = [&](V *p, int r, const uint32_t (&gr)[4]) { return p + ((uint64_t)reg_sum<RB>(r, gr) << LOW); };
+    {
+        V *p = thread_at(P.gin_t);
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
-            uint64_t ro = 0;
-#pragma unroll
-            for (int j = 0; j < RB; ++j) ro += (r >> j & 1) ? P.gin_r[j] : 0ull;
-            const V x = p[ro];
+            const V x = *reg_at(p, r, P.gin_r);
             v.r[r] = x.x;
             v.i[r] = x.y;
         }
     }
     // the ladders' factors, while the loads are in flight
-    V *lane_f = tile + (1u << P.K), *warp_f = lane_f + 32 * P.nladders;
+    V *lane_f = tile + tile_slots<T>(P.K), *warp_f = lane_f + 32 * P.nladders;
+    const uint32_t lw = P.K - RB - 5;                          // log2 of the CTA's warps
     if (P.nladders) {
-        const uint32_t lw = P.K - RB - 5;                      // log2 of the CTA's warps
         for (uint32_t i = t; i < 32u * P.nladders; i += blockDim.x) {
             double fr, fi;
             ladder_lane(P, i >> 5, i & 31, fr, fi);
@@ -52,12 +56,18 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
         }
         __syncthreads();
     }
+    auto factor = [&](uint32_t l, T &fr, T &fi) {
+        const V x = lane_f[32 * l + (t & 31)], y = warp_f[(l << lw) + (t >> 5)];
+        fr = x.x;
+        fi = x.y;
+        cmul(fr, fi, y.x, y.y);
+    };
     uint32_t slot = 0;
     for (int s = 0; s < P.nstages; ++s) {
         const Stage &st = P.st[s];
         uint32_t tt = 0;
 #pragma unroll
-        for (int j = 0; j < kMaxThreadBits; ++j) tt ^= (t >> j & 1) ? st.tb[j] : 0u;
+        for (int j = 0; j < kMaxThreadBits; ++j) tt += (t >> j & 1) * st.tb[j];
         if (s) {
             // to the new stage's registers through shared memory.  The slots
             // written are the ones this thread read at the stage before, so
@@ -66,15 +76,16 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
             uint32_t pr[4];
 #pragma unroll
             for (int j = 0; j < RB; ++j) pr[j] = sp.pr[j];
+            V *w = tile + slot;
 #pragma unroll
-            for (int r = 0; r < NR; ++r) tile[slot ^ reg_xor<RB>(r, pr)] = V{v.r[r], v.i[r]};
+            for (int r = 0; r < NR; ++r) w[reg_sum<RB>(r, pr)] = V{v.r[r], v.i[r]};
             __syncthreads();
-            slot = tt >> 16;
 #pragma unroll
             for (int j = 0; j < RB; ++j) pr[j] = st.pr[j];
+            w = tile + (tt >> 16);
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
-                const V x = tile[slot ^ reg_xor<RB>(r, pr)];
+                const V x = w[reg_sum<RB>(r, pr)];
                 v.r[r] = x.x;
                 v.i[r] = x.y;
             }
@@ -84,23 +95,14 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
         const int end = st.first + st.count;
         for (int o = st.first; o < end; ++o) {
             const Op<T> &op = P.op[o];
-            if ((base & op.need) != op.need) continue;         // the same for the whole CTA
-            if ((ti & op.cthr) != op.cthr) continue;
-            T fr = 1, fi = 0;
-            if (op.kind >= K_LADR && op.kind <= K_LAD0) {
-                const uint32_t lw = P.K - RB - 5;
-                const V x = lane_f[32 * op.ladder + (t & 31)], y = warp_f[(op.ladder << lw) + (t >> 5)];
-                fr = x.x;
-                fi = x.y;
-                cmul(fr, fi, y.x, y.y);
+            if (op.cond) {
+                if ((base & op.need) != op.need) continue;     // the same for the whole CTA
+                if ((ti & op.cthr) != op.cthr) continue;
             }
-            apply_op<T, RB>(v, op, fr, fi);
+            apply_op<T, RB>(v, op, factor);
         }
     }
     {
-        uint64_t off = base;
-#pragma unroll
-        for (int j = 0; j < kMaxThreadBits; ++j) off |= (t >> j & 1) ? P.gout_t[j] : 0ull;
         if (P.scale_kind == 1) {
 #pragma unroll
             for (int r = 0; r < NR; ++r) { v.r[r] *= P.scale[0]; v.i[r] *= P.scale[0]; }
@@ -108,28 +110,23 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
 #pragma unroll
             for (int r = 0; r < NR; ++r) cmul(v.r[r], v.i[r], P.scale[0], P.scale[1]);
         }
-        V *p = pa + off;
+        V *p = thread_at(P.gout_t);
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            uint64_t ro = 0;
-#pragma unroll
-            for (int j = 0; j < RB; ++j) ro += (r >> j & 1) ? P.gout_r[j] : 0ull;
-            p[ro] = V{v.r[r], v.i[r]};
-        }
+        for (int r = 0; r < NR; ++r) *reg_at(p, r, P.gout_r) = V{v.r[r], v.i[r]};
     }
 }
 
 template <typename T, typename R>
 int launch(qs_state *s, const R &P)
 {
-    const size_t amps = (1ull << P.K) + (size_t)P.nladders * (32 + (1u << (P.K - Traits<T>::RB - 5)));
+    const size_t amps = tile_slots<T>(P.K) + (size_t)P.nladders * (32 + (1u << (P.K - Traits<T>::RB - 5)));
     const size_t smem = 2 * sizeof(T) * amps;
     if (smem > 48 * 1024) {
         // once per device and kernel: the largest a pass can need
         static std::atomic<uint64_t> done{0};
         const uint64_t bit = 1ull << (s->device & 63);
         if (!(done.load() & bit)) {
-            const int most = (int)(2 * sizeof(T) * ((1u << kMaxTile) + R::NLAD * (32 + (1u << (kMaxTile - Traits<T>::RB - 5)))));
+            const int most = (int)(2 * sizeof(T) * (tile_slots<T>(kMaxTile) + R::NLAD * (32 + (1u << (kMaxTile - Traits<T>::RB - 5)))));
             QS_CUDA_TRY(cudaFuncSetAttribute(k_stage<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
             done.fetch_or(bit);
         }

@@ -13,7 +13,8 @@
 //
 // What the planner (qs_stage_plan.cpp) does to the gate list, all of it exact
 // algebra on the gates:
-//  - 1-qubit gates that follow each other on a qubit are multiplied in FP64;
+//  - 1-qubit gates that follow each other on a qubit are multiplied in FP64
+//    where the product keeps their form, or three or more follow;
 //  - a real or RX-like 1-qubit matrix is taken as p * [[1, r], [q, +-1]] with
 //    its largest row entry p pulled out: 4 multiply-adds per amplitude pair
 //    instead of 16; the p's of a pass are collected (FP64, on the host) and
@@ -24,14 +25,16 @@
 //  - gates that commute (no shared qubit, or diagonal on every shared one)
 //    may be taken out of order when that fills a pass or a stage.
 //
-// Shared memory is XOR-swizzled by a linear map: tile bit b >= LB adds the
-// LB-bit vector kVec[b] to the slot's low LB bits (LB = log2 of the
-// amplitudes per 128-byte row: 4 for complex64, 3 for complex128).  Any 4
-// register bits leave thread bits whose LB-bit images span all LB dimensions
-// (the images of the K <= 13 bits are distinct nonzero vectors for LB = 4,
-// each used at most twice for LB = 3: a code of distance > 4), and each stage
-// orders its lane bits so that the first LB are independent: every access
-// phase hits distinct banks.
+// Shared memory is padded, and additive: tile bit b weighs slot_weight(b)
+// slots, 2^b for the bits of one 128-byte row and, row digit by row digit, a
+// number that is 2^(b mod LB) modulo the row (LB = log2 of the amplitudes per
+// 128-byte row: 4 for complex64, 3 for complex128).  An amplitude's slot is
+// then the sum of a thread's part and a register's part, the second the same
+// for all threads: no instruction per access goes into addresses (an XOR
+// swizzle took one, on the pipe that was full).  Lanes whose LB first bits
+// differ modulo LB hit distinct banks; a stage orders its lane bits so,
+// which fails only when the registers take all of a residue class (3 or 4
+// tile bits), and then costs a second wavefront.
 #pragma once
 
 #include <cmath>
@@ -83,7 +86,8 @@ enum Kind : uint8_t {
     K_LADR = 47,     // ladder on the registers with every bit of creg
     K_LAD = 48,      // ladder on the registers with bit j set
     K_LAD0 = 52,     // ladder on every register
-    K_EX = 53        // dense 2x2 on (r | bit ja, r | bit jb), ja < jb, where creg is set: 53 + pair index
+    K_EX = 53,       // dense 2x2 on (r | bit ja, r | bit jb), ja < jb, where creg is set: 53 + pair index
+    K_XC = 60        // exchange x and y of register bit j where register bit c is set: 60 + 4 c + j
 };
 
 template <typename T>
@@ -91,7 +95,8 @@ struct Op {
     uint8_t kind;
     uint8_t creg;                // register-index bits that must be set
     uint16_t cthr;               // tile-index bits (thread bits of the stage) that must be set
-    uint32_t ladder;             // K_LAD*: index of its tables
+    uint16_t cond;               // need or cthr is not empty
+    uint16_t ladder;             // K_LAD*: index of its tables
     uint64_t need;               // state-index bits outside the tile that must be set
     T m[8];                      // dense: 2x2 row-major complex; pivot kinds: r, q; phase: one complex;
                                  // ladder: one complex per register bit
@@ -99,8 +104,8 @@ struct Op {
 
 struct Stage {
     uint16_t first, count;                 // its ops
-    uint16_t pr[4];                        // slot offset of register bit j
-    uint32_t tb[kMaxThreadBits];           // thread bit j: tile offset | slot offset << 16
+    uint16_t pr[4];                        // slot weight of register bit j
+    uint32_t tb[kMaxThreadBits];           // thread bit j: tile offset | slot weight << 16
 };
 
 // One ladder: the phases w of its entries multiply where the entry's bit is
@@ -125,8 +130,10 @@ struct Run {
     int32_t scale_kind;                    // 0: none, 1: real, 2: complex
     int32_t pad;
     uint64_t seg_mask[kMaxSeg];            // the tile index's bits, segment by segment ...
-    uint64_t gin_t[kMaxThreadBits], gin_r[4];      // state offsets of the load's thread and register bits
-    uint64_t gout_t[kMaxThreadBits], gout_r[4];    // ... and of the store's
+    // state offsets, in units of 2^LOW amplitudes, of the load's and the store's
+    // thread bits from LOW up (the first LOW are qubits 0..LOW-1) and register bits
+    uint32_t gin_t[kMaxThreadBits], gin_r[4];
+    uint32_t gout_t[kMaxThreadBits], gout_r[4];
     uint8_t seg_shift[kMaxSeg + 3];        // ... shifted left by this
     Stage st[NST_];
     Ladder lad[NLAD_];
@@ -138,20 +145,23 @@ template <typename T> using RunLarge = Run<T, 208, 56, 16, 256>;
 static_assert(sizeof(RunLarge<double>) <= 32764, "kernel parameters are at most 32764 bytes");
 
 // ------------------------------------------------------------------ index maps
+// the weight of tile bit b in shared-memory slots: digit d of base 2^LB
+// strides 1, 17, 273 (complex64) or 1, 9, 73, 585 (complex128), each past the
+// largest sum of the digits below it
 template <typename T>
-constexpr uint32_t bit_image(int b)
+constexpr uint32_t slot_weight(int b)
 {
-    // the vectors of tile bits >= LB (bits below LB: their own)
-    constexpr uint8_t v4[12] = {3, 5, 6, 9, 10, 12, 7, 11, 13, 14, 15, 15};
-    constexpr uint8_t v3[12] = {3, 5, 6, 7, 1, 2, 4, 3, 5, 6, 7, 7};
-    return b < Traits<T>::LB ? 1u << b : Traits<T>::LB == 4 ? v4[b - 4] : v3[b - 3];
+    constexpr uint32_t stride4[3] = {1, 17, 273}, stride3[4] = {1, 9, 73, 585};
+    return (Traits<T>::LB == 4 ? stride4[b / 4] : stride3[b / 3]) << (b % Traits<T>::LB);
 }
 
-// the shared-memory slot of tile index 2^b
+// slots of a K-bit tile
 template <typename T>
-constexpr uint32_t bit_slot(int b)
+constexpr uint32_t tile_slots(int K)
 {
-    return b < Traits<T>::LB ? 1u << b : (1u << b) | bit_image<T>(b);
+    uint32_t n = 1;
+    for (int b = 0; b < K; ++b) n += slot_weight<T>(b);
+    return n;
 }
 
 template <typename R>
@@ -163,10 +173,10 @@ QS_HD uint64_t tile_base(const R &P, uint64_t tl)
 }
 
 template <int RB>
-QS_HD uint32_t reg_xor(int r, const uint32_t (&b)[4])
+QS_HD uint32_t reg_sum(int r, const uint32_t (&b)[4])
 {
     uint32_t o = 0;
-    for (int j = 0; j < RB; ++j) o ^= (r >> j & 1) ? b[j] : 0u;
+    for (int j = 0; j < RB; ++j) o += (r >> j & 1) ? b[j] : 0u;
     return o;
 }
 
@@ -179,23 +189,72 @@ struct Regs {
 QS_HD float f_ma(float a, float b, float c) { return fmaf(a, b, c); }
 QS_HD double f_ma(double a, double b, double c) { return fma(a, b, c); }
 
-template <typename T>
-QS_HD void cmul(T &xr, T &xi, T pr, T pi)
-{
-    const T x = xr, y = xi;
-    xr = f_ma(x, pr, -(y * pi));
-    xi = f_ma(x, pi, y * pr);
-}
+// The updates of an amplitude pair, x and y on one component or on both.  On
+// the device each is one asm statement that reads its values and writes them
+// back in place, so that every case of apply_op leaves all registers where it
+// found them: as plain expressions the compiler kept the cases' results apart
+// and copied every amplitude after each op, about 100 moves an op (12 RY
+// gates, 28 qubits complex64: 1.64 ms, with the statements 1.33 ms).
+#ifdef __CUDA_ARCH__
+#define QS_UPD_T(NAME, T, C, S, BODY)                                                                              \
+    __device__ __forceinline__ void NAME(T &x, T &y, T r, T q)                                                     \
+    {                                                                                                              \
+        asm volatile("{\n\t.reg ." S " t, u;\n\t" BODY(S) "mov." S " %0, t;\n\t}" : "+" C(x), "+" C(y) : C(r), C(q)); \
+    }
+#define QS_UPD(NAME, BODY, HOST) QS_UPD_T(NAME, float, "f", "f32", BODY) QS_UPD_T(NAME, double, "d", "f64", BODY)
+#else
+#define QS_UPD(NAME, BODY, HOST) \
+    template <typename T> inline void NAME(T &x, T &y, T r, T q) { const T x0 = x, y0 = y; HOST; }
+#endif
+#define QS_B_AP(t) "fma.rn." t " t, %2, %1, %0;\n\tfma.rn." t " %1, %3, %0, %1;\n\t"
+#define QS_B_AM(t) "fma.rn." t " t, %2, %1, %0;\n\tneg." t " u, %1;\n\tfma.rn." t " %1, %3, %0, u;\n\t"
+#define QS_B_BP(t) "fma.rn." t " t, %2, %0, %1;\n\tfma.rn." t " %1, %3, %1, %0;\n\t"
+#define QS_B_BM(t) "fma.rn." t " t, %2, %0, %1;\n\tneg." t " u, %0;\n\tfma.rn." t " %1, %3, %1, u;\n\t"
+#define QS_B_BN(t) "neg." t " u, %1;\n\tfma.rn." t " t, %2, %0, u;\n\tfma.rn." t " %1, %3, %1, %0;\n\t"
+#define QS_B_MUL(t) "mul.rn." t " t, %1, %3;\n\tneg." t " t, t;\n\tfma.rn." t " t, %0, %2, t;\n\t" \
+                    "mul.rn." t " u, %0, %3;\n\tfma.rn." t " %1, %1, %2, u;\n\t"
+#define QS_B_SWAP(t) "mov." t " t, %1;\n\tmov." t " %1, %0;\n\t"
+QS_UPD(upd_ap, QS_B_AP, (x = f_ma(r, y0, x0), y = f_ma(q, x0, y0)))
+QS_UPD(upd_am, QS_B_AM, (x = f_ma(r, y0, x0), y = f_ma(q, x0, -y0)))
+QS_UPD(upd_bp, QS_B_BP, (x = f_ma(r, x0, y0), y = f_ma(q, y0, x0)))
+QS_UPD(upd_bm, QS_B_BM, (x = f_ma(r, x0, y0), y = f_ma(q, y0, -x0)))
+QS_UPD(upd_bn, QS_B_BN, (x = f_ma(r, x0, -y0), y = f_ma(q, y0, x0)))
+QS_UPD(cmul, QS_B_MUL, (x = f_ma(x0, r, -(y0 * q)), y = f_ma(y0, r, x0 * q)))      // (x + iy)(r + iq)
+QS_UPD(upd_swap4, QS_B_SWAP, (x = y0, y = x0, (void)r, (void)q))
 
 template <typename T>
-QS_HD void dense2(T &ar, T &ai, T &br, T &bi, const T *m)
+QS_HD void upd_swap(T &x, T &y) { upd_swap4(x, y, (T)0, (T)0); }
+
+#ifdef __CUDA_ARCH__
+#define QS_DENSE(T, C, t)                                                                                         \
+    __device__ __forceinline__ void dense2(T &xr, T &xi, T &yr, T &yi, const T *m)                                \
+    {                                                                                                             \
+        asm volatile("{\n\t.reg ." t " a, b, c, d, n;\n\t"                                                        \
+                     "mul.rn." t " a, %4, %0;\n\tmul.rn." t " b, %4, %1;\n\t"                                     \
+                     "mul.rn." t " c, %8, %0;\n\tmul.rn." t " d, %8, %1;\n\t"                                     \
+                     "fma.rn." t " b, %5, %0, b;\n\tfma.rn." t " d, %9, %0, d;\n\t"                               \
+                     "neg." t " n, %1;\n\tfma.rn." t " a, %5, n, a;\n\tfma.rn." t " c, %9, n, c;\n\t"             \
+                     "fma.rn." t " a, %6, %2, a;\n\tfma.rn." t " b, %6, %3, b;\n\t"                               \
+                     "fma.rn." t " c, %10, %2, c;\n\tfma.rn." t " d, %10, %3, d;\n\t"                             \
+                     "fma.rn." t " b, %7, %2, b;\n\tfma.rn." t " d, %11, %2, d;\n\t"                              \
+                     "neg." t " n, %3;\n\tfma.rn." t " a, %7, n, a;\n\tfma.rn." t " c, %11, n, c;\n\t"            \
+                     "mov." t " %0, a;\n\tmov." t " %1, b;\n\tmov." t " %2, c;\n\tmov." t " %3, d;\n\t}"          \
+                     : "+" C(xr), "+" C(xi), "+" C(yr), "+" C(yi)                                                 \
+                     : C(m[0]), C(m[1]), C(m[2]), C(m[3]), C(m[4]), C(m[5]), C(m[6]), C(m[7]));                   \
+    }
+QS_DENSE(float, "f", "f32")
+QS_DENSE(double, "d", "f64")
+#else
+template <typename T>
+inline void dense2(T &ar, T &ai, T &br, T &bi, const T *m)
 {
     const T xr = ar, xi = ai, yr = br, yi = bi;
-    ar = f_ma(-m[3], yi, f_ma(m[2], yr, f_ma(-m[1], xi, m[0] * xr)));
+    ar = f_ma(m[3], -yi, f_ma(m[2], yr, f_ma(m[1], -xi, m[0] * xr)));
     ai = f_ma(m[3], yr, f_ma(m[2], yi, f_ma(m[1], xr, m[0] * xi)));
-    br = f_ma(-m[7], yi, f_ma(m[6], yr, f_ma(-m[5], xi, m[4] * xr)));
+    br = f_ma(m[7], -yi, f_ma(m[6], yr, f_ma(m[5], -xi, m[4] * xr)));
     bi = f_ma(m[7], yr, f_ma(m[6], yi, f_ma(m[5], xr, m[4] * xi)));
 }
+#endif
 
 template <typename T, int RB, int J, int KIND>
 QS_HD void op_pair(Regs<T, RB> &v, const T *m, uint32_t creg)
@@ -206,38 +265,31 @@ QS_UNROLL
         for (int a = 0; a < (1 << RB); ++a) {
             if (a >> J & 1) continue;
             const int b = a | 1 << J;
-            T xr = v.r[a], xi = v.i[a], yr = v.r[b], yi = v.i[b];
+            T &xr = v.r[a], &xi = v.i[a], &yr = v.r[b], &yi = v.i[b];
             if constexpr (KIND == K_RAP) {
-                v.r[a] = f_ma(r, yr, xr); v.i[a] = f_ma(r, yi, xi);
-                v.r[b] = f_ma(q, xr, yr); v.i[b] = f_ma(q, xi, yi);
+                upd_ap(xr, yr, r, q); upd_ap(xi, yi, r, q);
             } else if constexpr (KIND == K_RAM) {
-                v.r[a] = f_ma(r, yr, xr); v.i[a] = f_ma(r, yi, xi);
-                v.r[b] = f_ma(q, xr, -yr); v.i[b] = f_ma(q, xi, -yi);
+                upd_am(xr, yr, r, q); upd_am(xi, yi, r, q);
             } else if constexpr (KIND == K_RBP) {
-                v.r[a] = f_ma(r, xr, yr); v.i[a] = f_ma(r, xi, yi);
-                v.r[b] = f_ma(q, yr, xr); v.i[b] = f_ma(q, yi, xi);
+                upd_bp(xr, yr, r, q); upd_bp(xi, yi, r, q);
             } else if constexpr (KIND == K_RBM) {
-                v.r[a] = f_ma(r, xr, yr); v.i[a] = f_ma(r, xi, yi);
-                v.r[b] = f_ma(q, yr, -xr); v.i[b] = f_ma(q, yi, -xi);
+                upd_bm(xr, yr, r, q); upd_bm(xi, yi, r, q);
             } else if constexpr (KIND == K_IA) {
-                v.r[a] = f_ma(-r, yi, xr); v.i[a] = f_ma(r, yr, xi);
-                v.r[b] = f_ma(-q, xi, yr); v.i[b] = f_ma(q, xr, yi);
+                upd_ap(xr, yi, -r, q); upd_ap(xi, yr, r, -q);
             } else if constexpr (KIND == K_IB) {
-                v.r[a] = f_ma(r, xr, -yi); v.i[a] = f_ma(r, xi, yr);
-                v.r[b] = f_ma(q, yr, -xi); v.i[b] = f_ma(q, yi, xr);
+                upd_bn(xr, yi, r, q); upd_bm(xi, yr, r, q);
             } else if constexpr (KIND == K_GEN) {
-                dense2(v.r[a], v.i[a], v.r[b], v.i[b], m);
+                dense2(xr, xi, yr, yi, m);
             } else if constexpr (KIND == K_GENR) {
-                if ((a & creg) == creg) dense2(v.r[a], v.i[a], v.r[b], v.i[b], m);
+                if ((a & creg) == creg) dense2(xr, xi, yr, yi, m);
             } else if constexpr (KIND == K_X) {
-                v.r[a] = yr; v.i[a] = yi;
-                v.r[b] = xr; v.i[b] = xi;
+                upd_swap(xr, yr); upd_swap(xi, yi);
             } else if constexpr (KIND == K_XR) {
-                const bool on = (a & creg) == creg;
-                v.r[a] = on ? yr : xr; v.i[a] = on ? yi : xi;
-                v.r[b] = on ? xr : yr; v.i[b] = on ? xi : yi;
+                if ((a & creg) == creg) { upd_swap(xr, yr); upd_swap(xi, yi); }
+            } else if constexpr (KIND >= K_XC) {
+                if (a >> ((KIND - K_XC) / 4) & 1) { upd_swap(xr, yr); upd_swap(xi, yi); }
             } else {                                        // K_PH
-                cmul(v.r[b], v.i[b], m[0], m[1]);
+                cmul(yr, yi, m[0], m[1]);
             }
         }
     }
@@ -278,10 +330,10 @@ QS_HD void ladder_walk(Regs<T, RB> &v, T fr, T fi, const T *m, uint32_t creg)
     }
 }
 
-// One op on a thread's registers (its need and cthr hold).  fr + i fi: a
-// ladder's factor for this thread.
-template <typename T, int RB>
-QS_HD void apply_op(Regs<T, RB> &v, const Op<T> &op, T fr, T fi)
+// One op on a thread's registers (its need and cthr hold).  factor(ladder,
+// fr, fi) gives a ladder's factor for this thread.
+template <typename T, int RB, typename F>
+QS_HD void apply_op(Regs<T, RB> &v, const Op<T> &op, const F &factor)
 {
     const T *m = op.m;
     const uint32_t creg = op.creg;
@@ -316,14 +368,30 @@ QS_UNROLL
 QS_UNROLL
         for (int a = 0; a < (1 << RB); ++a) { v.r[a] *= m[0]; v.i[a] *= m[0]; }
         break;
-    case K_LADR: ladder_walk<T, RB, RB, RB - 1, 0>(v, fr, fi, m, creg); break;
-    case K_LAD + 0: ladder_walk<T, RB, 0, RB - 1, 0>(v, fr, fi, m, creg); break;
-    case K_LAD + 1: ladder_walk<T, RB, 1, RB - 1, 0>(v, fr, fi, m, creg); break;
-    case K_LAD + 2: ladder_walk<T, RB, 2, RB - 1, 0>(v, fr, fi, m, creg); break;
-    case K_LAD + 3:
-        if constexpr (RB > 3) ladder_walk<T, RB, 3, RB - 1, 0>(v, fr, fi, m, creg);
+#define QS_STG_LAD(KIND, HUB)                                                     \
+    case KIND:                                                                    \
+        if constexpr (HUB < RB || KIND == K_LADR) {                               \
+            T fr, fi;                                                             \
+            factor(op.ladder, fr, fi);                                            \
+            ladder_walk<T, RB, HUB, RB - 1, 0>(v, fr, fi, m, creg);               \
+        }                                                                         \
         break;
-    case K_LAD0: ladder_walk<T, RB, -2, RB - 1, 0>(v, fr, fi, m, creg); break;
+    QS_STG_LAD(K_LADR, RB)
+    QS_STG_LAD(K_LAD + 0, 0)
+    QS_STG_LAD(K_LAD + 1, 1)
+    QS_STG_LAD(K_LAD + 2, 2)
+    QS_STG_LAD(K_LAD + 3, 3)
+    QS_STG_LAD(K_LAD0, -2)
+#undef QS_STG_LAD
+#define QS_STG_XC(C)                                                              \
+    QS_STG_XCJ(C, 0) QS_STG_XCJ(C, 1) QS_STG_XCJ(C, 2) QS_STG_XCJ(C, 3)
+#define QS_STG_XCJ(C, J)                                                          \
+    case K_XC + 4 * C + J:                                                        \
+        if constexpr (C < RB && C != J) op_pair<T, RB, J, K_XC + 4 * C>(v, m, creg); \
+        break;
+    QS_STG_XC(0) QS_STG_XC(1) QS_STG_XC(2) QS_STG_XC(3)
+#undef QS_STG_XCJ
+#undef QS_STG_XC
     case K_EX + 0: op_exchange<T, RB, 0, 1>(v, m, creg); break;
     case K_EX + 1: op_exchange<T, RB, 0, 2>(v, m, creg); break;
     case K_EX + 2: op_exchange<T, RB, 1, 2>(v, m, creg); break;
@@ -358,7 +426,7 @@ QS_HD void ladder_warp(const R &P, int l, uint32_t warp, uint64_t base, double &
 
 // ------------------------------------------------------------------ planner (qs_stage_plan.cpp)
 // One operation of the simplified gate list.
-enum GType : uint8_t { G_U, G_CU, G_EX, G_SWAP, G_DIAG };
+enum GType : uint8_t { G_NONE, G_U, G_CU, G_EX, G_SWAP, G_DIAG };
 struct GOp {
     uint8_t type;
     uint64_t tgt;                // qubits it mixes: they must be tile qubits
@@ -367,7 +435,6 @@ struct GOp {
     uint64_t off0, off1;         // G_EX: the exchanged qubits
     double m[8];                 // G_U, G_CU, G_EX: 2x2; G_DIAG: m[0] + i m[1] a factor of every amplitude
     int first, count;            // G_DIAG: its terms [first, first + count) in Planner::terms
-    int prim, nprims;            // the gates it stands for, when they are nprims = 1: prims[prim]
 };
 struct Term {
     int q;                       // the phase applies where the hub and this qubit are set (-1: the hub alone)

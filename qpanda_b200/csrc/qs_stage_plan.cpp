@@ -21,6 +21,15 @@ bool is_x(const double m[8])
 
 bool is_diag(const double m[8]) { return m[2] == 0 && m[3] == 0 && m[4] == 0 && m[5] == 0; }
 
+// diagonal, real, real diagonal with imaginary rest (RX), or none of these
+int form(const double m[8])
+{
+    if (is_diag(m)) return 0;
+    if (m[1] == 0 && m[3] == 0 && m[5] == 0 && m[7] == 0) return 1;
+    if (m[1] == 0 && m[7] == 0 && m[2] == 0 && m[4] == 0) return 2;
+    return 3;
+}
+
 // a := b * a, 2x2 row-major complex
 void mul2(double a[8], const double b[8])
 {
@@ -41,30 +50,43 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
     K = n < kMaxTile ? n : kMaxTile;
     low = dtype == QS_C64 ? Traits<float>::LOW : Traits<double>::LOW;
     ops.reserve(prims.size());
-    int open[64];                          // the 1-qubit op that a gate on this qubit may join
-    for (int &o : open) o = -1;
+    // the 1-qubit ops at the end of a qubit's list: the last one and, when
+    // nothing else lies between, the one before it
+    int open[64], before[64];
+    for (int q = 0; q < 64; ++q) open[q] = before[q] = -1;
     int last_diag = -1;                    // the phase op that another phase may join ...
     uint64_t since = 0;                    // ... and the qubits mixed after it
     for (size_t i = 0; i < prims.size(); ++i) {
         const qs_prim &p = prims[i];
         if (p.kind == QS_PRIM_PAIR && p.off0 == 0 && p.cmask == 0) {
-            const int q = low_bit(p.off1);
-            if (open[q] >= 0) {
-                mul2(ops[open[q]].m, p.m);
-                ++ops[open[q]].nprims;
+            // Gates of one form multiply into one op.  Two of different forms
+            // stay two ops: their product would be dense, 20 instructions per
+            // pair against 6 + 5 for a rotation and a phase; three become one.
+            const int q = low_bit(p.off1), o = open[q];
+            if (o >= 0 && (form(ops[o].m) == form(p.m) || form(ops[o].m) == 3)) {
+                mul2(ops[o].m, p.m);
+                continue;
+            }
+            if (o >= 0 && before[q] >= 0) {
+                GOp &g = ops[before[q]];
+                mul2(g.m, ops[o].m);
+                mul2(g.m, p.m);
+                ops[o].type = G_NONE;
+                open[q] = before[q];
+                before[q] = -1;
                 continue;
             }
             GOp g = {};
             g.type = G_U;
             g.tgt = p.off1;
             memcpy(g.m, p.m, sizeof(g.m));
-            g.nprims = 1;
+            before[q] = o;
             open[q] = (int)ops.size();
             since |= g.tgt;
             ops.push_back(g);
             continue;
         }
-        for (uint64_t h = p.holes; h; h &= h - 1) open[low_bit(h)] = -1;
+        for (uint64_t h = p.holes; h; h &= h - 1) open[low_bit(h)] = before[low_bit(h)] = -1;
         if (p.kind == QS_PRIM_PHASE) {
             if (last_diag >= 0 && !(since & p.holes)) {
                 // join the last phase op when every term then has at most one
@@ -79,7 +101,6 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
                     d.diag |= p.holes;
                     terms.push_back({mine ? low_bit(mine) : -1, p.m[0], p.m[1]});
                     ++d.count;
-                    ++d.nprims;
                     continue;
                 }
             }
@@ -89,7 +110,6 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
             g.m[0] = 1;
             g.first = (int)terms.size();
             g.count = 1;
-            g.nprims = 1;
             terms.push_back({-1, p.m[0], p.m[1]});
             last_diag = (int)ops.size();
             since = 0;
@@ -98,7 +118,6 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
         }
         GOp g = {};
         memcpy(g.m, p.m, sizeof(g.m));
-        g.nprims = 1;
         g.ctrl = g.diag = p.cmask;
         if (p.off0 == 0) {
             g.type = G_CU;
@@ -130,8 +149,9 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
         g.tgt = 0;
         g.type = G_DIAG;
     }
-    left.resize(ops.size());
-    for (size_t i = 0; i < ops.size(); ++i) left[i] = (int)i;
+    left.reserve(ops.size());
+    for (size_t i = 0; i < ops.size(); ++i)
+        if (ops[i].type != G_NONE) left.push_back((int)i);
 }
 
 // Ops of `left` that can run in a pass on the tile of q: their targets in q,
@@ -370,19 +390,16 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         return regs;
     };
     // the stage's layout; lanes: the tile bits that must come first, in order
-    int thread_of[kMaxTile], reg_of[kMaxTile];
+    int thread_of[kMaxTile], reg_of[kMaxTile], reg_at[4], reg_in[4];
     auto add_stage = [&](uint32_t regs, const int *lanes, int nlanes) {
         Stage &st = S.st[S.nstages++];
         memset(&st, 0, sizeof(st));
         st.first = (uint16_t)nops;
         int order[kMaxTile], no = 0;
-        uint32_t basis[4] = {0, 0, 0, 0}, used = regs;
-        auto independent = [&](int b) {
-            uint32_t v = bit_image<T>(b);
-            for (int h = LB - 1; h >= 0; --h)
-                if ((v >> h & 1) && basis[h]) v ^= basis[h];
-            if (!v) return false;
-            basis[31 - __builtin_clz(v)] = v;
+        uint32_t classes = 0, used = regs;
+        auto independent = [&](int b) {                // another residue class of the row's banks
+            if (classes >> (b % LB) & 1) return false;
+            classes |= 1u << (b % LB);
             return true;
         };
         for (int j = 0; j < nlanes; ++j) {
@@ -399,13 +416,14 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
             if (!(used >> b & 1)) order[no++] = b;
         for (int b = 0; b < K; ++b) thread_of[b] = reg_of[b] = -1;
         for (int j = 0; j < tbits; ++j) {
-            st.tb[j] = (1u << order[j]) | bit_slot<T>(order[j]) << 16;
+            st.tb[j] = (1u << order[j]) | slot_weight<T>(order[j]) << 16;
             thread_of[order[j]] = j;
         }
         int j = 0;
         for (int b = 0; b < K; ++b)
             if (regs >> b & 1) {
-                st.pr[j] = (uint16_t)bit_slot<T>(b);
+                st.pr[j] = (uint16_t)slot_weight<T>(b);
+                reg_at[j] = b;
                 reg_of[b] = j++;
             }
         return &st;
@@ -422,6 +440,7 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
                 if (reg_of[b] >= 0) op->creg |= 1u << reg_of[b];
                 else op->cthr |= 1u << b;
             }
+        op->cond = op->need || op->cthr;
     };
     auto reg_bit = [&](uint64_t qs) { return reg_of[pos[low_bit(qs)]]; };
     // one op at the current stage; false when it does not fit the parameter block
@@ -442,7 +461,9 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
             condition(g.ctrl, &op);
             for (int k = 0; k < 8; ++k) op.m[k] = (T)g.m[k];
             const bool x = is_x(g.m);
-            op.kind = (uint8_t)((x ? (op.creg ? K_XR : K_X) : (op.creg ? K_GENR : K_GEN)) + reg_bit(g.tgt));
+            const bool one = op.creg && !(op.creg & (op.creg - 1));
+            op.kind = (uint8_t)((x ? (one ? K_XC + 4 * low_bit(op.creg) : op.creg ? K_XR : K_X) : op.creg ? K_GENR : K_GEN) +
+                                reg_bit(g.tgt));
         } else if (g.type == G_EX) {
             condition(g.ctrl, &op);
             int ja = reg_bit(g.off0), jb = reg_bit(g.off1);
@@ -459,7 +480,7 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
             if (S.nladders == R::NLAD || nent + g.count > R::NENT) return false;
             condition(g.ctrl, &op);
             for (int j = 0; j < RB; ++j) op.m[2 * j] = 1;
-            op.ladder = (uint32_t)S.nladders;
+            op.ladder = (uint16_t)S.nladders;
             Ladder &L = S.lad[S.nladders++];
             L.first = (uint16_t)nent;
             L.nthr = L.nout = L.pad = 0;
@@ -518,6 +539,7 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         // every thread must then store where it loaded
         if (first && last) last = memcmp(ps, pos, sizeof(int) * (size_t)n) == 0;
         Stage *st = add_stage(regs, first ? natural : lanes, first || last ? LOW : 0);
+        if (first) memcpy(reg_in, reg_at, sizeof(reg_in));
         size_t k = 0, t = 0;
         for (; k < take.size(); ++k)
             if (!emit(P.ops[(size_t)take[k]])) {
@@ -553,12 +575,12 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
     int at[kMaxTile];                              // qubit behind a tile bit at the store
     for (int q = 0; q < n; ++q)
         if (pos[q] >= 0) at[pos[q]] = q;
-    auto offsets = [&](const Stage &st, const int *qs, uint64_t *gt, uint64_t *gr) {
-        for (int j = 0; j < tbits; ++j) gt[j] = 1ull << qs[low_bit(st.tb[j] & 0xffffu)];
-        for (int j = 0; j < RB; ++j) gr[j] = 1ull << qs[31 - __builtin_clz((uint32_t)st.pr[j])];
+    auto offsets = [&](const Stage &st, const int *regs, const int *qs, uint32_t *gt, uint32_t *gr) {
+        for (int j = LOW; j < tbits; ++j) gt[j] = 1u << (qs[low_bit(st.tb[j] & 0xffffu)] - LOW);
+        for (int j = 0; j < RB; ++j) gr[j] = 1u << (qs[regs[j]] - LOW);
     };
-    offsets(S.st[0], qubit, S.gin_t, S.gin_r);
-    offsets(S.st[S.nstages - 1], at, S.gout_t, S.gout_r);
+    offsets(S.st[0], reg_in, qubit, S.gin_t, S.gin_r);
+    offsets(S.st[S.nstages - 1], reg_at, at, S.gout_t, S.gout_r);
     S.scale[0] = (T)scale.real();
     S.scale[1] = (T)scale.imag();
     S.scale_kind = scale.imag() != 0 ? 2 : scale.real() != 1 ? 1 : 0;

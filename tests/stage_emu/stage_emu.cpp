@@ -57,18 +57,19 @@ template <typename T, typename R>
 int run_pass(std::vector<V2<T>> &a, int n, const R &P, Stats &st)
 {
     constexpr int RB = Traits<T>::RB, NR = 1 << RB;
-    const uint32_t threads = 1u << (P.K - RB), TN = 1u << P.K;
+    const uint32_t threads = 1u << (P.K - RB);
     if (P.nstages < 1 || P.nstages > R::NST || P.nladders > R::NLAD) return fail("stages %lld", P.nstages);
     std::vector<uint8_t> seen(a.size(), 0), stored(a.size(), 0);
-    std::vector<V2<T>> tile(TN), out(a);
+    const uint32_t slots_n = tile_slots<T>(P.K);
+    std::vector<V2<T>> tile(slots_n), out(a);
     std::vector<Regs<T, RB>> v(threads);
     for (uint64_t tl = 0; tl < a.size() >> P.K; ++tl) {
         const uint64_t base = tile_base(P, tl);
-        auto offset = [&](uint32_t t, int r, const uint64_t *gt, const uint64_t *gr) {
-            uint64_t o = base;
-            for (int j = 0; j < kMaxThreadBits; ++j) o |= (t >> j & 1) ? gt[j] : 0;
-            for (int j = 0; j < RB; ++j) o += (r >> j & 1) ? gr[j] : 0;
-            return o;
+        auto offset = [&](uint32_t t, int r, const uint32_t *gt, const uint32_t (&gr)[4]) {
+            constexpr int LOW = Traits<T>::LOW;
+            uint64_t u = reg_sum<RB>(r, gr);
+            for (int j = LOW; j < kMaxThreadBits; ++j) u += (t >> j & 1) * gt[j];
+            return base + (t & ((1u << LOW) - 1)) + (u << LOW);
         };
         for (uint32_t t = 0; t < threads; ++t)
             for (int r = 0; r < NR; ++r) {
@@ -83,18 +84,18 @@ int run_pass(std::vector<V2<T>> &a, int n, const R &P, Stats &st)
             std::vector<uint32_t> prev(tt);
             for (uint32_t t = 0; t < threads; ++t) {
                 tt[t] = 0;
-                for (int j = 0; j < kMaxThreadBits; ++j) tt[t] ^= (t >> j & 1) ? sg.tb[j] : 0u;
+                for (int j = 0; j < kMaxThreadBits; ++j) tt[t] += (t >> j & 1) * sg.tb[j];
             }
             if (s) {
-                std::vector<uint8_t> wr(TN, 0), rd(TN, 0);
+                std::vector<uint8_t> wr(slots_n, 0), rd(slots_n, 0);
                 for (int write = 1; write >= 0; --write) {
                     uint32_t pr[4];
                     for (int j = 0; j < 4; ++j) pr[j] = write ? P.st[s - 1].pr[j] : sg.pr[j];
                     for (int r = 0; r < NR; ++r) {
                         std::vector<uint32_t> slots(threads);
                         for (uint32_t t = 0; t < threads; ++t) {
-                            const uint32_t sl = ((write ? prev[t] : tt[t]) >> 16) ^ reg_xor<RB>(r, pr);
-                            if (sl >= TN || (write ? wr : rd)[sl]++) return fail("slot %lld used twice", sl);
+                            const uint32_t sl = ((write ? prev[t] : tt[t]) >> 16) + reg_sum<RB>(r, pr);
+                            if (sl >= slots_n || (write ? wr : rd)[sl]++) return fail("slot %lld used twice", sl);
                             if (write) tile[sl] = {v[t].r[r], v[t].i[r]};
                             else { v[t].r[r] = tile[sl].x; v[t].i[r] = tile[sl].y; }
                             slots[t] = sl;
@@ -106,20 +107,19 @@ int run_pass(std::vector<V2<T>> &a, int n, const R &P, Stats &st)
             for (int o = sg.first; o < sg.first + sg.count; ++o) {
                 if (o >= R::NOP) return fail("op %lld past the block", o);
                 const Op<T> &op = P.op[o];
+                if (op.kind >= K_LADR && op.kind <= K_LAD0 && op.ladder >= P.nladders) return fail("ladder %lld", op.ladder);
+                if (!op.cond && (op.need || op.cthr)) return fail("op %lld hides its condition", o);
                 if ((base & op.need) != op.need) continue;
                 for (uint32_t t = 0; t < threads; ++t) {
                     if ((tt[t] & op.cthr) != op.cthr) continue;
-                    T fr = 1, fi = 0;
-                    if (op.kind >= K_LADR && op.kind <= K_LAD0) {
-                        if ((int)op.ladder >= P.nladders) return fail("ladder %lld", op.ladder);
+                    apply_op<T, RB>(v[t], op, [&](uint32_t l, T &fr, T &fi) {
                         double lr, li, wr, wi;
-                        ladder_lane(P, op.ladder, t & 31, lr, li);
-                        ladder_warp(P, op.ladder, t >> 5, base, wr, wi);
+                        ladder_lane(P, l, t & 31, lr, li);
+                        ladder_warp(P, l, t >> 5, base, wr, wi);
                         fr = (T)lr;
                         fi = (T)li;
                         cmul(fr, fi, (T)wr, (T)wi);
-                    }
-                    apply_op<T, RB>(v[t], op, fr, fi);
+                    });
                 }
             }
         }
