@@ -72,13 +72,24 @@ struct BatchCirc {
     const LoadMap *loads;        // their tile-order copy maps
     const qs_tmem::TLayout *tlayouts;   // its passes' tensor-memory layouts (k_batch_tmem), or null
     double *zz;                  // nq - 1 outputs
-    int32_t npass, nq, nq_eff, pad;
+    // a circuit that is shared among CTAs, in parts of `part` tiles (k_batch_tmem; else nparts = 0)
+    int32_t *done;               // parts finished so far, over all passes
+    double *norms;               // [npass][nparts] output norms of the parts
+    double *zzp;                 // [nparts][kMaxZZ] unnormalised <ZZ> sums of the parts
+    int32_t npass, nq, nq_eff, nparts, part, pad;
+};
+
+// What a CTA of k_batch_tmem takes from the queue: a whole circuit (pass < 0)
+// or one part of one pass of a shared circuit.
+struct BatchTask {
+    int32_t circ, pass, part;
 };
 
 struct BatchParams {
     const BatchCirc *circ;
-    const int32_t *order;        // processing order (longest first)
-    int32_t ncirc;
+    const int32_t *order;        // processing order (longest first): k_batch
+    const BatchTask *tasks;      // k_batch_tmem
+    int32_t ncirc, ntasks;
     int32_t *head;               // queue position, zeroed before the launch
     int *err;
 };
@@ -334,6 +345,16 @@ __global__ void __launch_bounds__(kThreads, BShape<SUB>::kCtasPerSm) k_batch(Bat
 // is: the queue, |0...0> on the first pass without reading memory, the
 // previous pass's norm folded into the first block's matrix, and the
 // <Z_i Z_{i+1}> of the last pass's output.
+//
+// A circuit that would keep one CTA busy past the others' end is shared: its
+// passes are cut into parts of a few tiles, each a task of the queue.  A part
+// of pass p waits until all parts of pass p - 1 are done.  They precede it in
+// the queue, so a CTA only ever waits for tasks that running CTAs have taken:
+// the earliest unfinished task never waits, whatever number of CTAs is
+// resident.  Norms and <ZZ> sums are added part by part in a fixed order.
+// (256 circuits of 10..22 qubits, 4..12 layers: one CTA per circuit took what
+// the deepest 22-qubit circuit takes, 96.6 ms; shared, 8.9 ms with the same
+// bits.  16 circuits of 20..22 qubits: 96.7 -> 3.9 ms.)
 constexpr int kTmThreads = 128;
 constexpr int kTmCtasPerSm = 3;
 constexpr uint32_t kTmOffB = 0;                                      // 2 blocks x (hi, lo) x 8 KB
@@ -346,6 +367,31 @@ constexpr uint32_t kTmCols = 128;
 static_assert(kTmCtasPerSm * (kTmSmemBytes + 1024) <= 228 * 1024, "resident CTAs per SM");
 static_assert(kTmCtasPerSm * kTmCols <= 512, "TMEM columns per SM");
 static_assert((4 + 4 * kMaxZZ) * 8 <= kStage, "reductions fit the staging buffer");
+
+// a warp's sum of n values that other CTAs wrote, in a fixed order
+__device__ __forceinline__ double sum_parts(const double *v, int stride, int n)
+{
+    double s = 0;
+    for (int k = threadIdx.x & 31; k < n; k += 32) s += __ldcg(v + (size_t)k * stride);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// Wait until `need` parts of a circuit are done; false when that took longer
+// than any task can (2 s) or another CTA has failed.
+__device__ bool wait_parts(const int32_t *done, int32_t need, const int *err)
+{
+    uint64_t t0 = 0, now;
+    for (uint32_t spin = 0;; ++spin) {
+        int32_t v;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
+        if (v >= need) return true;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        if (spin == 0) t0 = now;
+        if (now - t0 > 2000000000ull || *reinterpret_cast<const volatile int *>(err)) return false;
+        __nanosleep(100);
+    }
+}
 
 __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchParams P)
 {
@@ -382,15 +428,15 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
     bool failed = false;
 
     while (!failed) {
-        if (tid == 0) {
-            const int c = atomicAdd(P.head, 1);
-            *s_circ = c < P.ncirc ? P.order[c] : -1;
-        }
+        if (tid == 0) *s_circ = atomicAdd(P.head, 1);
         __syncthreads();
-        const int ci = *s_circ;
-        if (ci < 0) break;
-        const BatchCirc C = P.circ[ci];
-        const uint64_t tiles = 1ull << (C.nq_eff - 12);
+        if (*s_circ >= P.ntasks) break;
+        const BatchTask task = P.tasks[*s_circ];
+        const BatchCirc C = P.circ[task.circ];
+        const bool shared = task.pass >= 0;
+        const uint64_t all_tiles = 1ull << (C.nq_eff - 12);
+        const uint64_t tile0 = shared ? (uint64_t)task.part * C.part : 0;
+        const uint64_t tiles = shared && tile0 + C.part < all_tiles ? tile0 + C.part : all_tiles;   // one past the last
         const int nzz = C.nq - 1;
         float scale = 1.0f;
         double zz[kMaxZZ];
@@ -398,11 +444,18 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
         for (int i = 0; i < kMaxZZ; ++i) zz[i] = 0.0;
         double out_norm = 0.0;
 
-        for (int p = 0; p < C.npass && !failed; ++p) {
+        const int p_end = shared ? task.pass + 1 : C.npass;
+        for (int p = shared ? task.pass : 0; p < p_end && !failed; ++p) {
             {
                 const uint32_t *src = reinterpret_cast<const uint32_t *>(C.tlayouts + p);
                 uint32_t *dst = reinterpret_cast<uint32_t *>(&L);
                 for (int i = tid; i < (int)(sizeof(qs_tmem::TLayout) / 4); i += kTmThreads) dst[i] = src[i];
+            }
+            if (shared && p > 0) {
+                // the parts of the previous pass, and their norm
+                if (__syncthreads_or(tid == 0 && !wait_parts(C.done, p * C.nparts, P.err))) { failed = true; break; }
+                const double norm = sum_parts(C.norms + (size_t)(p - 1) * C.nparts, 1, C.nparts);
+                scale = norm > 0 ? (float)(1.0 / sqrt(norm)) : 1.0f;
             }
             __syncthreads();
             D::load_b_perm(smem + kTmOffB, C.mats + (size_t)C.layouts[p].pad * 2 * 64 * 64, L, scale);
@@ -436,9 +489,9 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
             const bool last_pass = p + 1 == C.npass;
             double acc_out = 0;
             const uint64_t step = D::tbase_of(1, L);
-            uint64_t tbase = 0;
+            uint64_t tbase = shared ? D::tbase_of(tile0, L) : 0;
             if (p > 0) D::copy_tile<1>(C.amp, tbase, L, stage, g_t, cs_t);
-            for (uint64_t tile = 0; tile < tiles; ++tile) {
+            for (uint64_t tile = tile0; tile < tiles; ++tile) {
                 const uint64_t tnext = tile_base_advance(tbase, step, L.tmask);
                 float y[64];
                 if (p == 0) {
@@ -535,16 +588,36 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
             __syncthreads();
         }
         if (failed) break;
+        const bool final_pass = !shared || task.pass + 1 == C.npass;
+        if (final_pass) {
 #pragma unroll
-        for (int i = 0; i < kMaxZZ; ++i)
-            for (int o = 16; o > 0; o >>= 1) zz[i] += __shfl_xor_sync(0xffffffffu, zz[i], o);
-        if (lane == 0)
+            for (int i = 0; i < kMaxZZ; ++i)
+                for (int o = 16; o > 0; o >>= 1) zz[i] += __shfl_xor_sync(0xffffffffu, zz[i], o);
+            if (lane == 0)
 #pragma unroll
-            for (int i = 0; i < kMaxZZ; ++i) red[4 + warp * kMaxZZ + i] = zz[i];
-        __syncthreads();
-        for (int i = tid; i < nzz; i += kTmThreads)
-            C.zz[i] = (red[4 + i] + red[4 + kMaxZZ + i] + red[4 + 2 * kMaxZZ + i] + red[4 + 3 * kMaxZZ + i]) /
-                      out_norm;
+                for (int i = 0; i < kMaxZZ; ++i) red[4 + warp * kMaxZZ + i] = zz[i];
+            __syncthreads();
+            for (int i = tid; i < nzz; i += kTmThreads) {
+                const double sum = red[4 + i] + red[4 + kMaxZZ + i] + red[4 + 2 * kMaxZZ + i] + red[4 + 3 * kMaxZZ + i];
+                if (shared) C.zzp[(size_t)task.part * kMaxZZ + i] = sum;
+                else C.zz[i] = sum / out_norm;
+            }
+        }
+        if (shared) {
+            if (tid == 0) C.norms[(size_t)task.pass * C.nparts + task.part] = out_norm;
+            __threadfence();                                 // this part's stores, before it counts as done
+            __syncthreads();
+            if (tid == 0) *s_circ = atomicAdd(C.done, 1) + 1;
+            __syncthreads();
+            if (*s_circ == C.npass * C.nparts) {             // the circuit's last part: its <ZZ>
+                __threadfence();
+                const double norm = sum_parts(C.norms + (size_t)task.pass * C.nparts, 1, C.nparts);
+                for (int i = warp; i < nzz; i += kTmThreads / 32) {
+                    const double sum = sum_parts(C.zzp + i, kMaxZZ, C.nparts);
+                    if (lane == 0) C.zz[i] = sum / norm;
+                }
+            }
+        }
         __syncthreads();
     }
     if (failed) {
@@ -578,8 +651,11 @@ struct qs_batch {
     bool use_tmem = false;
     void *d_circ = nullptr;              // BatchCirc[n]
     void *d_order = nullptr;
+    void *d_tasks = nullptr;             // BatchTask[ntasks] (k_batch_tmem)
+    double *d_parts = nullptr;           // shared circuits' norms and <ZZ> sums
+    int32_t ntasks = 0, nshared = 0;
     double *d_zz = nullptr;
-    int32_t *d_head = nullptr;           // queue head + error flag
+    int32_t *d_head = nullptr;           // queue head, error flag, the shared circuits' counters
     size_t zz_count = 0, state_bytes = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
@@ -593,7 +669,7 @@ void batch_free(qs_batch *B)
     if (B->graph_exec) cudaGraphExecDestroy(B->graph_exec);
     if (B->graph) cudaGraphDestroy(B->graph);
     for (void *p : {B->d_states, B->d_mats, B->d_layouts, B->d_loads, B->d_tlayouts, B->d_circ, B->d_order,
-                    (void *)B->d_zz, (void *)B->d_head})
+                    B->d_tasks, (void *)B->d_parts, (void *)B->d_zz, (void *)B->d_head})
         if (p) cudaFree(p);
     delete B;
 }
@@ -608,6 +684,59 @@ std::string signature(int nq, const qs_gate *g, size_t count)
         s.append(reinterpret_cast<const char *>(g[i].ctrl), sizeof(int32_t) * (size_t)std::max(0, g[i].nctrl));
     }
     return s;
+}
+
+// The queue of k_batch_tmem for `ctas` resident CTAs.  A circuit is shared
+// when alone it would take more than half of an even share of the work (in
+// tiles x passes): below that, longest-first over whole circuits ends within
+// that half.  All shared circuits run in step, by the passes they have left
+// (the deepest start first and all end together), in parts of so many tiles
+// that a step gives every CTA about two; whole circuits fill steps with fewer
+// parts than CTAs, the rest follow.  A part costs its block matrices' load
+// once more (32 KB from L2), so it has at least 2 tiles.  Returns the doubles
+// that the shared circuits need; their norms / zzp get offsets into them.
+size_t plan_tasks(std::vector<BatchCirc> &hc, const std::vector<int32_t> &order, int ctas,
+                  std::vector<BatchTask> *tasks, int32_t *nshared)
+{
+    auto tiles = [&](const BatchCirc &c) { return (int64_t)1 << (c.nq_eff - 12); };
+    int64_t total = 0, shared_tiles = 0;
+    for (const BatchCirc &c : hc) total += c.npass * tiles(c);
+    std::vector<int32_t> shared, whole;
+    int deepest = 0;
+    for (int32_t i : order) {
+        const BatchCirc &c = hc[(size_t)i];
+        if (tiles(c) >= 4 && c.npass > 0 && 2 * ctas * c.npass * tiles(c) > total) {
+            shared.push_back(i);
+            shared_tiles += tiles(c);
+            deepest = std::max(deepest, (int)c.npass);
+        } else {
+            whole.push_back(i);
+        }
+    }
+    const int64_t per = shared_tiles < 8 * (int64_t)ctas ? ctas : 2 * (int64_t)ctas;
+    const int32_t part = (int32_t)std::max<int64_t>(2, (shared_tiles + per - 1) / per);
+    size_t doubles = 0;
+    for (int32_t i : shared) {
+        BatchCirc &c = hc[(size_t)i];
+        c.part = part;
+        c.nparts = (int32_t)((tiles(c) + part - 1) / part);
+        c.norms = reinterpret_cast<double *>(doubles);
+        doubles += (size_t)c.npass * c.nparts;
+        c.zzp = reinterpret_cast<double *>(doubles);
+        doubles += (size_t)kMaxZZ * c.nparts;
+    }
+    size_t w = 0;
+    for (int left = deepest; left > 0; --left) {
+        const size_t from = tasks->size();
+        for (int32_t i : shared) {
+            const BatchCirc &c = hc[(size_t)i];
+            for (int32_t k = 0; c.npass >= left && k < c.nparts; ++k) tasks->push_back({i, c.npass - left, k});
+        }
+        for (; w < whole.size() && tasks->size() - from < (size_t)ctas; ++w) tasks->push_back({whole[w], -1, 0});
+    }
+    for (; w < whole.size(); ++w) tasks->push_back({whole[w], -1, 0});
+    *nshared = (int32_t)shared.size();
+    return doubles;
 }
 
 }  // namespace
@@ -775,7 +904,6 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
         if (e == cudaSuccess) e = cudaMalloc(&B->d_circ, sizeof(BatchCirc) * n_circ);
         if (e == cudaSuccess) e = cudaMalloc(&B->d_order, sizeof(int32_t) * n_circ);
         if (e == cudaSuccess) e = cudaMalloc((void **)&B->d_zz, std::max<size_t>(B->zz_count, 1) * sizeof(double));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&B->d_head, 2 * sizeof(int32_t));
         // The block matrices as BF16: a run of consecutive circuits at a time
         // is converted on the host threads into one of two pinned buffers
         // while the other's copy to the device is in flight.
@@ -842,6 +970,9 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
             bc.npass = (int32_t)pp->passes.size();
             bc.nq = B->nq[c];
             bc.nq_eff = B->nq_eff[c];
+            bc.done = nullptr;
+            bc.norms = bc.zzp = nullptr;
+            bc.nparts = bc.part = bc.pad = 0;
         }
         // processing order: longest first (tiles x passes), or as given
         B->order.resize(n_circ);
@@ -851,7 +982,24 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
                 return (double)hc[a].npass * (double)(1ull << hc[a].nq_eff) >
                        (double)hc[b].npass * (double)(1ull << hc[b].nq_eff);
             });
-        e = cudaMemcpy(B->d_circ, hc.data(), sizeof(BatchCirc) * n_circ, cudaMemcpyHostToDevice);
+        std::vector<BatchTask> tasks;
+        if (B->use_tmem) {
+            const size_t doubles = plan_tasks(hc, B->order, QS_SM_COUNT * kTmCtasPerSm, &tasks, &B->nshared);
+            B->ntasks = (int32_t)tasks.size();
+            e = cudaMalloc((void **)&B->d_parts, std::max<size_t>(doubles, 1) * sizeof(double));
+            if (e == cudaSuccess) e = cudaMalloc(&B->d_tasks, std::max<size_t>(tasks.size(), 1) * sizeof(BatchTask));
+            if (e == cudaSuccess && !tasks.empty())
+                e = cudaMemcpy(B->d_tasks, tasks.data(), tasks.size() * sizeof(BatchTask), cudaMemcpyHostToDevice);
+        }
+        if (e == cudaSuccess) e = cudaMalloc((void **)&B->d_head, (2 + (size_t)B->nshared) * sizeof(int32_t));
+        // the shared circuits' buffers: plan_tasks left offsets in their place
+        for (int c = 0, k = 0; c < n_circ && e == cudaSuccess; ++c) {
+            if (!hc[c].nparts) continue;
+            hc[c].done = B->d_head + 2 + k++;
+            hc[c].norms = B->d_parts + (size_t)hc[c].norms;
+            hc[c].zzp = B->d_parts + (size_t)hc[c].zzp;
+        }
+        if (e == cudaSuccess) e = cudaMemcpy(B->d_circ, hc.data(), sizeof(BatchCirc) * n_circ, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(B->d_order, B->order.data(), sizeof(int32_t) * n_circ, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) r = qs_cuda_fail(e, "qs_batch_create: tables");
     }
@@ -866,15 +1014,17 @@ namespace {
 
 int batch_launch(qs_batch *B, cudaStream_t st)
 {
-    QS_CUDA_TRY(cudaMemsetAsync(B->d_head, 0, 2 * sizeof(int32_t), st));
+    QS_CUDA_TRY(cudaMemsetAsync(B->d_head, 0, (2 + (size_t)B->nshared) * sizeof(int32_t), st));
     BatchParams P;
+    P.tasks = static_cast<const BatchTask *>(B->d_tasks);
+    P.ntasks = B->ntasks;
     P.circ = static_cast<const BatchCirc *>(B->d_circ);
     P.order = static_cast<const int32_t *>(B->d_order);
     P.ncirc = B->n;
     P.head = B->d_head;
     P.err = B->d_head + 1;
     if (B->use_tmem) {
-        const unsigned grid = (unsigned)std::min(B->n, QS_SM_COUNT * kTmCtasPerSm);
+        const unsigned grid = (unsigned)std::min(B->ntasks, QS_SM_COUNT * kTmCtasPerSm);
         k_batch_tmem<<<grid, kTmThreads, kTmSmemBytes, st>>>(P);
     } else if (B->opts.max_sub <= 2) {
         const unsigned grid = (unsigned)std::min(B->n, QS_SM_COUNT * BShape<2>::kCtasPerSm);

@@ -1,0 +1,35 @@
+"""Batches whose widest circuits are shared among CTAs (qs_batch.cu): one
+circuit alone at the smallest and at larger widths, a wide one beside many
+narrow ones, circuits of unequal depth in step.  <Z_i Z_{i+1}> against the
+FP64 oracle within the batch tests' tolerance (a complex64 state after fused
+tensor-core passes), states and replays of the graph with it."""
+import numpy as np
+import pytest
+
+from qpanda_b200 import Batch, circuits
+from tests.test_gpu_batch import TOL, oracle_zz
+
+pytestmark = pytest.mark.gpu
+
+SWEEPS = {
+    "alone_14": [(14, 3)],
+    "alone_18": [(18, 4)],
+    "wide_beside_narrow": [(19, 3)] + [(8 + k % 6, 1 + k % 4) for k in range(40)],
+    "unequal": [(17, 1), (16, 5), (18, 2), (14, 4), (17, 4)],
+}
+
+
+@pytest.mark.parametrize("name", list(SWEEPS))
+@pytest.mark.parametrize("order", [0, 1])
+def test_shared_circuits_match_oracle(need_gpu, name, order):
+    sweep = [(q, circuits.vqe_ansatz(q, layers, seed=100 * q + layers)) for q, layers in SWEEPS[name]]
+    b = Batch(sweep, order=order)
+    b.run()
+    zz = b.zz()
+    for _ in range(3):                       # the same bits every time, whichever CTA takes which part
+        b.run()
+        assert all(np.array_equal(a, c) for a, c in zip(zz, b.zz()))
+    for k, (q, g) in enumerate(sweep):
+        ref_zz, ref_state = oracle_zz(q, g)
+        assert np.abs(zz[k] - ref_zz).max() < TOL, (k, q)
+        assert np.abs(b.state(k) - ref_state).max() < TOL, (k, q)
