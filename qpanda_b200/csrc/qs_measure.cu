@@ -407,23 +407,58 @@ size_t marginal_smem(const MargParams &P)
 }
 
 // -------------------------------------------------------------- shots
-// tree[2^k + x] = P(first k measured outcomes = x) for k <= K0.
-__global__ void k_fold(double *tree, int k)
+// tree[2^k + x] = P(first k measured outcomes = x) for k <= K0; level k from
+// level k + 1: tree[2^k + x] = tree[2^(k+1) + x] + tree[2^(k+1) + x + 2^k].
+// One launch per level was most of a small sampler call (9 qubits, 256 shots:
+// 9 of 12 launches); here a CTA carries a set of columns through all levels it
+// can: k_fold_cols the levels K0 - 1 .. kFoldLow of a wide tree (16 columns a
+// CTA: 128-byte rows), k_fold_top the levels below, one CTA.
+constexpr int kFoldLow = 11;
+constexpr int kFoldCols = 16;
+
+__global__ void __launch_bounds__(kThreads) k_fold_cols(double *tree, int K0)
 {
-    const uint64_t n = 1ull << k;
-    double *dst = tree + n;
-    const double *src = tree + 2 * n;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += stride)
-        dst[x] = src[x] + src[x + n];
+    extern __shared__ double fold_sm[];                        // [2^(K0 - kFoldLow)][kFoldCols]
+    const uint64_t c0 = (uint64_t)blockIdx.x * kFoldCols;
+    for (uint32_t i = threadIdx.x; i < (uint32_t)kFoldCols << (K0 - kFoldLow); i += kThreads)
+        fold_sm[i] = tree[(1ull << K0) + c0 + i % kFoldCols + ((uint64_t)(i / kFoldCols) << kFoldLow)];
+    for (int k = K0 - 1; k >= kFoldLow; --k) {
+        const uint32_t half = (uint32_t)kFoldCols << (k - kFoldLow);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < half; i += kThreads) {
+            const double v = fold_sm[i] + fold_sm[i + half];
+            fold_sm[i] = v;
+            tree[(1ull << k) + c0 + i % kFoldCols + ((uint64_t)(i / kFoldCols) << kFoldLow)] = v;
+        }
+    }
 }
+
+__global__ void __launch_bounds__(1024) k_fold_top(double *tree, int K)
+{
+    __shared__ double sm[1 << kFoldLow];
+    for (uint32_t i = threadIdx.x; i < 1u << K; i += blockDim.x) sm[i] = tree[(1u << K) + i];
+    for (int k = K - 1; k >= 0; --k) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < 1u << k; i += blockDim.x) {
+            const double v = sm[i] + sm[i + (1u << k)];
+            sm[i] = v;
+            tree[(1u << k) + i] = v;
+        }
+    }
+}
+
+// What k_shots needs of the measured qubits, by value: no copies to wait for.
+constexpr int kTreeQubits = 20;
+struct ShotParams {
+    int8_t qubits[64];
+    Holes deep[QS_MAX_QUBITS - kTreeQubits];      // levels kTreeQubits..: the qubits measured up to there
+};
 
 // One warp per shot.  Levels k < K0 read the tree; deeper levels sum the
 // amplitudes that match the outcomes so far (2^(n-k-1) of them).
 template <typename T>
 __global__ void k_shots(const T *__restrict__ a, const double *__restrict__ tree, int K0, int m,
-                        const Holes *__restrict__ deep, const int *__restrict__ qubits,
-                        const double *__restrict__ u, uint64_t shots, int n,
+                        const __grid_constant__ ShotParams P, const double *__restrict__ u, uint64_t shots, int n,
                         uint64_t *__restrict__ out)
 {
     typedef typename vec2<T>::type V;
@@ -439,7 +474,7 @@ __global__ void k_shots(const T *__restrict__ a, const double *__restrict__ tree
             if (k < K0) {
                 L = tree[(2ull << k) + x];
             } else {
-                const Holes &h = deep[k - K0];
+                const Holes &h = P.deep[k - K0];
                 const uint64_t cnt = 1ull << (n - k - 1);
                 double acc = 0;
                 for (uint64_t w = lane; w < cnt; w += 32) {
@@ -455,7 +490,7 @@ __global__ void k_shots(const T *__restrict__ a, const double *__restrict__ tree
             const double sc = 1.0 / sqrt(psel);
             S *= sc * sc;
             x |= (uint64_t)b << k;
-            F |= (uint64_t)b << qubits[k];
+            F |= (uint64_t)b << P.qubits[k];
         }
         if (lane == 0) out[s] = x;
     }
@@ -735,16 +770,12 @@ int probs_t(qs_state *s, const int *qubits, int m, double *out)
 template <typename T>
 int sample_t(qs_state *s, const int *qubits, int m, const double *u, size_t shots, uint64_t *out)
 {
-    const int K0 = m < 20 ? m : 20;
+    const int K0 = m < kTreeQubits ? m : kTreeQubits;
     const size_t tree_b = 16ull << K0;            // 2^(K0+1) doubles
     const size_t u_b = 8ull * shots * (size_t)m;
     const size_t out_b = 8ull * shots;
-    const int ndeep = m - K0;
-    const size_t deep_b = sizeof(Holes) * (size_t)(ndeep > 0 ? ndeep : 1);
-    const size_t q_b = 4ull * (m > 0 ? m : 1);
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    size_t o_tree = kBufOff, o_u = o_tree + al(tree_b), o_out = o_u + al(u_b),
-           o_deep = o_out + al(out_b), o_q = o_deep + al(deep_b), o_part = o_q + al(q_b);
+    size_t o_tree = kBufOff, o_u = o_tree + al(tree_b), o_out = o_u + al(u_b), o_part = o_out + al(out_b);
     size_t part_b = 0;
     MargParams P = marginal_plan(s, qubits, K0, &part_b);
     // Size scratch once, before any pointer into it is taken.
@@ -754,28 +785,27 @@ int sample_t(qs_state *s, const int *qubits, int m, const double *u, size_t shot
     double *tree = reinterpret_cast<double *>(sc + o_tree);
     // Level K0 = marginal over the first K0 measured qubits, stored at tree + 2^K0.
     if ((r = marginal_launch<T>(s, P, tree + (1ull << K0), reinterpret_cast<double *>(sc + o_part)))) return r;
-    for (int k = K0 - 1; k >= 0; --k) {
-        k_fold<<<grid_for(1ull << k, kThreads), kThreads, 0, s->stream>>>(tree, k);
-        QS_LAUNCH_CHECK("k_fold");
+    if (K0 > kFoldLow) {
+        const size_t smem = sizeof(double) * ((size_t)kFoldCols << (K0 - kFoldLow));     // 64 KB at most
+        QS_CUDA_TRY(cudaFuncSetAttribute(k_fold_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+        k_fold_cols<<<(1u << kFoldLow) / kFoldCols, kThreads, smem, s->stream>>>(tree, K0);
+        QS_LAUNCH_CHECK("k_fold_cols");
     }
-    std::vector<Holes> deep((size_t)(ndeep > 0 ? ndeep : 0));
+    k_fold_top<<<1, K0 < kFoldLow ? 256 : 1024, 0, s->stream>>>(tree, K0 < kFoldLow ? K0 : kFoldLow);
+    QS_LAUNCH_CHECK("k_fold_top");
+    ShotParams SP;
+    for (int k = 0; k < m; ++k) SP.qubits[k] = (int8_t)qubits[k];
     for (int k = K0; k < m; ++k) {
         uint64_t mask = 0;
         for (int j = 0; j <= k; ++j) mask |= 1ull << qubits[j];
-        deep[(size_t)(k - K0)] = holes_from_mask(mask);
+        SP.deep[k - K0] = holes_from_mask(mask);
     }
     QS_CUDA_TRY(cudaMemcpyAsync(sc + o_u, u, u_b, cudaMemcpyHostToDevice, s->stream));
-    if (ndeep > 0)
-        QS_CUDA_TRY(cudaMemcpyAsync(sc + o_deep, deep.data(), sizeof(Holes) * deep.size(),
-                                    cudaMemcpyHostToDevice, s->stream));
-    QS_CUDA_TRY(cudaMemcpyAsync(sc + o_q, qubits, 4ull * m, cudaMemcpyHostToDevice, s->stream));
     const int thr = 256;
     uint64_t warps_needed = shots;
     unsigned grid = (unsigned)std::min<uint64_t>((warps_needed * 32 + thr - 1) / thr, (uint64_t)QS_SM_COUNT * 8);
     if (grid < 1) grid = 1;
-    k_shots<T><<<grid, thr, 0, s->stream>>>(static_cast<const T *>(s->amp), tree, K0, m,
-                                            reinterpret_cast<const Holes *>(sc + o_deep),
-                                            reinterpret_cast<const int *>(sc + o_q),
+    k_shots<T><<<grid, thr, 0, s->stream>>>(static_cast<const T *>(s->amp), tree, K0, m, SP,
                                             reinterpret_cast<const double *>(sc + o_u), shots, s->n,
                                             reinterpret_cast<uint64_t *>(sc + o_out));
     QS_LAUNCH_CHECK("k_shots");
