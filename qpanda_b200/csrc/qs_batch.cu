@@ -451,14 +451,16 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                 uint32_t *dst = reinterpret_cast<uint32_t *>(&L);
                 for (int i = tid; i < (int)(sizeof(qs_tmem::TLayout) / 4); i += kTmThreads) dst[i] = src[i];
             }
+            __syncthreads();
+            D::BWords<kTmThreads, 2> words;
+            D::fetch_b(words, C.mats + (size_t)C.layouts[p].pad * 2 * 64 * 64, L);
             if (shared && p > 0) {
                 // the parts of the previous pass, and their norm
                 if (__syncthreads_or(tid == 0 && !wait_parts(C.done, p * C.nparts, P.err))) { failed = true; break; }
                 const double norm = sum_parts(C.norms + (size_t)(p - 1) * C.nparts, 1, C.nparts);
                 scale = norm > 0 ? (float)(1.0 / sqrt(norm)) : 1.0f;
             }
-            __syncthreads();
-            D::load_b_perm(smem + kTmOffB, C.mats + (size_t)C.layouts[p].pad * 2 * 64 * 64, L, scale);
+            D::store_b(words, smem + kTmOffB, L, scale);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();

@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 
 #include "../../include/qpanda_b200.h"
 
@@ -112,6 +113,36 @@ inline unsigned grid_for(uint64_t items, int threads, int blocks_per_sm = 16)
     if (b < 1) b = 1;
     return (unsigned)b;
 }
+
+// Launch a kernel that may start before the one ahead of it in the stream has
+// ended (programmatic dependent launch).  The kernel must call
+// qs_wait_previous() before it touches anything that earlier work on the
+// stream reads or writes; what comes before that call - setting up, fetching
+// what no earlier kernel writes - overlaps the other kernel's end, and the
+// gap between the two launches goes.
+template <typename... KArgs, typename... Args>
+cudaError_t qs_launch_overlapped(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                                 cudaStream_t stream, Args &&...args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, std::forward<Args>(args)...);
+}
+
+#ifdef __CUDACC__
+// the next kernel may be scheduled as CTAs of this one leave room
+__device__ __forceinline__ void qs_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// everything before this kernel on the stream has ended and is visible
+__device__ __forceinline__ void qs_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
 
 // ------------------------------------------------------------------ kernels API
 // (qs_gates.cu)

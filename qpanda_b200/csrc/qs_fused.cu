@@ -335,8 +335,11 @@ __global__ void __launch_bounds__(kFixThreads) k_norm_fix(float4 *amp, uint64_t 
                                                           const double *nlp, int nparts)
 {
     __shared__ float s_c;
+    qs_let_next_start();
+    qs_wait_previous();
     if (threadIdx.x < 32) {
         double a = 0.0, b = 0.0;
+#pragma unroll 8
         for (int i = threadIdx.x; i < nparts; i += 32) { a += n0p[i]; b += nlp[i]; }
         for (int o = 16; o > 0; o >>= 1) {
             a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -367,8 +370,8 @@ __global__ void __launch_bounds__(kFixThreads) k_norm_fix(float4 *amp, uint64_t 
 int qs_launch_norm_fix(qs_state *s, const double *norm0, const double *last_out, int nparts)
 {
     if (s->dtype != QS_C64) return QS_OK;
-    k_norm_fix<<<QS_SM_COUNT * 4, kFixThreads, 0, s->stream>>>(static_cast<float4 *>(s->amp), s->N / 2, norm0,
-                                                              last_out, nparts);
+    QS_CUDA_TRY(qs_launch_overlapped(k_norm_fix, grid_for(s->N / 2, kFixThreads, 4), kFixThreads, 0, s->stream,
+                                     static_cast<float4 *>(s->amp), s->N / 2, norm0, last_out, nparts));
     QS_LAUNCH_CHECK("k_norm_fix");
     return QS_OK;
 }

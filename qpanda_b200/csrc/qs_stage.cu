@@ -20,6 +20,7 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
     V *pa = reinterpret_cast<V *>(a);
     constexpr int LOW = Traits<T>::LOW;
     const uint32_t t = threadIdx.x;
+    qs_let_next_start();
     const uint64_t base = tile_base(P, blockIdx.x);
     Regs<T, RB> v;
     // the state address of a thread's register r: thread part + register part
@@ -33,6 +34,7 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
     auto reg_at = [&](V *p, int r, const uint32_t (&gr)[4]) { return p + ((uint64_t)reg_sum<RB>(r, gr) << LOW); };
     {
         V *p = thread_at(P.gin_t);
+        qs_wait_previous();
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             const V x = *reg_at(p, r, P.gin_r);
@@ -131,8 +133,8 @@ int launch(qs_state *s, const R &P)
             done.fetch_or(bit);
         }
     }
-    k_stage<T, R><<<(unsigned)(s->N >> P.K), 1u << (P.K - Traits<T>::RB), smem, s->stream>>>(static_cast<T *>(s->amp), P);
-    QS_LAUNCH_CHECK("k_stage");
+    QS_CUDA_TRY(qs_launch_overlapped(k_stage<T, R>, (unsigned)(s->N >> P.K), 1u << (P.K - Traits<T>::RB), smem,
+                                     s->stream, static_cast<T *>(s->amp), P));
     return QS_OK;
 }
 

@@ -23,6 +23,12 @@
 //      StoreMap).
 // The four groups' chains overlap each other on the SM.
 //
+// On small states a pass is its start and one chain per group.  The start is
+// kept off the chain: matrix words are fetched before the pass waits for the
+// one ahead of it (qs_wait_previous), the first tile's copies go out before the
+// norms are summed, and the launch itself overlaps the previous pass's end (21
+// qubits, 19 passes: 0.374 -> 0.294 ms; 16 qubits: 0.294 -> 0.208 ms).
+//
 // The previous pass's norm correction (a scalar) is folded into block 0's
 // matrix when the CTA loads it; the input norm is summed on the plan's first
 // pass only; every wait on an mbarrier is bounded (qs_tile::mbar_wait), and an
@@ -247,6 +253,7 @@ struct TParams {
     uint64_t tiles;
     const uint16_t *mat;         // nsub x [2][64][64] BF16 bits (hi, lo), the plan's column order
     int *err;
+    int early;                   // the next kernel may be scheduled from this one's start
     int nparts;                  // norm partials per pass (>= gridDim.x; the tail is written as zeros)
     const double *norm0;
     const double *prev_out;
@@ -274,6 +281,7 @@ __global__ void __launch_bounds__(TShape<TPR>::kCtaThreads, 1) k_tile_tmem(const
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + kOffMisc + 32);
     float *s_scale = reinterpret_cast<float *>(smem + kOffMisc + 36);
 
+    if (P.early) qs_let_next_start();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_u32(tmem_holder)), "r"(kCols));
@@ -283,27 +291,9 @@ __global__ void __launch_bounds__(TShape<TPR>::kCtaThreads, 1) k_tile_tmem(const
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(mbar)), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
-    if (warp == 1) {
-        double n0 = 0, np = 0;
-        if (P.norm0 && P.prev_out)
-            for (int i = lane; i < P.nparts; i += 32) { n0 += P.norm0[i]; np += P.prev_out[i]; }
-        for (int o = 16; o > 0; o >>= 1) {
-            n0 += __shfl_xor_sync(0xffffffffu, n0, o);
-            np += __shfl_xor_sync(0xffffffffu, np, o);
-        }
-        if (lane == 0) *s_scale = (P.norm0 && P.prev_out && np > 0) ? (float)sqrt(n0 / np) : 1.0f;
-    }
-    __syncthreads();
-    load_b_perm(smem + kOffB, P.mat, L, *s_scale);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *tmem_holder;
-    const uint32_t tgrp = tmem_base + (uint32_t)(grp * 128);          // the group's 128 columns
-    const uint32_t tlane = tgrp + ((uint32_t)(wq * 32) << 16);        // this warp's 32 lanes
-    const uint32_t mb = smem_u32(mbar);
-    const int bar_id = 1 + grp;
+    // the matrices' words, which no earlier pass writes
+    BWords<S::kCtaThreads, qs_tmem::kMaxSub> words;
+    fetch_b(words, P.mat, L);
 
     // per-thread parts of the gather, copy and store addresses
     uint32_t xrow = 0;
@@ -354,7 +344,31 @@ __global__ void __launch_bounds__(TShape<TPR>::kCtaThreads, 1) k_tile_tmem(const
     uint64_t tile = (uint64_t)blockIdx.x * kGroups + grp;
     const uint64_t step = tbase_of(stride, L);
     uint64_t tbase = tbase_of(tile, L);
+    qs_wait_previous();
     if (tile < P.tiles) copy_tile<TPR>(amp, tbase, L, stage, g_t, cs_t);
+    if (warp == 1) {
+        double n0 = 0, np = 0;
+        if (P.norm0 && P.prev_out) {
+#pragma unroll 8
+            for (int i = lane; i < P.nparts; i += 32) { n0 += P.norm0[i]; np += P.prev_out[i]; }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            n0 += __shfl_xor_sync(0xffffffffu, n0, o);
+            np += __shfl_xor_sync(0xffffffffu, np, o);
+        }
+        if (lane == 0) *s_scale = (P.norm0 && P.prev_out && np > 0) ? (float)sqrt(n0 / np) : 1.0f;
+    }
+    __syncthreads();
+    store_b(words, smem + kOffB, L, *s_scale);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_holder;
+    const uint32_t tgrp = tmem_base + (uint32_t)(grp * 128);          // the group's 128 columns
+    const uint32_t tlane = tgrp + ((uint32_t)(wq * 32) << 16);        // this warp's 32 lanes
+    const uint32_t mb = smem_u32(mbar);
+    const int bar_id = 1 + grp;
     for (; tile < P.tiles; tile += stride) {
         const uint64_t tnext = tile_base_advance(tbase, step, L.tmask);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -502,6 +516,9 @@ int qs_launch_tiled_tmem(qs_state *s, const qs_tiled_desc *d, int *err_dev)
     P.tiles = s->N >> 12;
     P.mat = static_cast<const uint16_t *>(d->mat_dev);
     P.err = err_dev;
+    // up to 25 qubits (24: 1.54 -> 1.51 ms for 31 passes; 21: 0.322 -> 0.294 ms
+    // for 19); at 30 the next pass's early CTAs cost 1 %
+    P.early = P.tiles <= 16ull * QS_SM_COUNT * kGroups;
     P.nparts = qs_tiled_grid(s);
     P.norm0 = d->norm0;
     P.prev_out = d->prev_out;
@@ -516,10 +533,10 @@ int qs_launch_tiled_tmem(qs_state *s, const qs_tiled_desc *d, int *err_dev)
     const unsigned grid = (unsigned)qs_tmem_grid(s);
     if (d->threads_per_row == 2) {
         QS_CUDA_TRY(cudaFuncSetAttribute(k_tile_tmem<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        k_tile_tmem<2><<<grid, TShape<2>::kCtaThreads, kSmemBytes, s->stream>>>(in, out, P);
+        QS_CUDA_TRY(qs_launch_overlapped(k_tile_tmem<2>, grid, TShape<2>::kCtaThreads, kSmemBytes, s->stream, in, out, P));
     } else {
         QS_CUDA_TRY(cudaFuncSetAttribute(k_tile_tmem<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        k_tile_tmem<1><<<grid, TShape<1>::kCtaThreads, kSmemBytes, s->stream>>>(in, out, P);
+        QS_CUDA_TRY(qs_launch_overlapped(k_tile_tmem<1>, grid, TShape<1>::kCtaThreads, kSmemBytes, s->stream, in, out, P));
     }
     QS_LAUNCH_CHECK("k_tile_tmem");
     return QS_OK;

@@ -46,17 +46,38 @@ __device__ __forceinline__ uint64_t tbase_of(uint64_t tile, const TLayout &L)
 // Block matrices into the swizzled B layout, each permuted to this kernel's
 // column order (register bit p = matrix bit mperm[b][p], for rows and
 // columns alike); block 0's scaled by `scale` (hi + lo recombined, scaled,
-// split again).
-__device__ inline void load_b_perm(uint8_t *dst, const uint16_t *mat, const TLayout &L, float scale)
+// split again).  In two steps, so that the words can be under way before the
+// scale is known: fetch_b reads this thread's words (item it = thread +
+// k threads of nsub 64 x 32 ones), store_b writes them.
+template <int NT, int NSUB>
+struct BWords {
+    static constexpr int kItems = NSUB * 64 * 32 / NT;
+    uint32_t hi[kItems], lo[kItems];
+};
+
+template <int NT, int NSUB>
+__device__ __forceinline__ void fetch_b(BWords<NT, NSUB> &w, const uint16_t *mat, const TLayout &L)
 {
-    const int total = L.nsub * 64 * 32;
-    for (int it = threadIdx.x; it < total; it += blockDim.x) {
-        const int b = it >> 11, np = (it >> 5) & 63, cp = it & 31;
+#pragma unroll
+    for (int k = 0; k < BWords<NT, NSUB>::kItems; ++k) {
+        const int it = threadIdx.x + k * NT, b = it >> 11, np = (it >> 5) & 63, cp = it & 31;
+        if (b >= L.nsub) break;
         const uint32_t n = 2 * qs_tmem::tmem_matrix_index((uint32_t)np >> 1, L.mperm[b]) + (np & 1);
-        const uint32_t k = 2 * qs_tmem::tmem_matrix_index((uint32_t)cp, L.mperm[b]);
+        const uint32_t c = 2 * qs_tmem::tmem_matrix_index((uint32_t)cp, L.mperm[b]);
         const uint16_t *src = mat + (size_t)b * 2 * 4096;
-        uint32_t hi = *reinterpret_cast<const uint32_t *>(src + n * 64 + k);
-        uint32_t lo = *reinterpret_cast<const uint32_t *>(src + 4096 + n * 64 + k);
+        w.hi[k] = *reinterpret_cast<const uint32_t *>(src + n * 64 + c);
+        w.lo[k] = *reinterpret_cast<const uint32_t *>(src + 4096 + n * 64 + c);
+    }
+}
+
+template <int NT, int NSUB>
+__device__ __forceinline__ void store_b(const BWords<NT, NSUB> &w, uint8_t *dst, const TLayout &L, float scale)
+{
+#pragma unroll
+    for (int k = 0; k < BWords<NT, NSUB>::kItems; ++k) {
+        const int it = threadIdx.x + k * NT, b = it >> 11, np = (it >> 5) & 63, cp = it & 31;
+        if (b >= L.nsub) break;
+        uint32_t hi = w.hi[k], lo = w.lo[k];
         if (b == 0 && scale != 1.0f) {
             const float a = (__uint_as_float(hi << 16) + __uint_as_float(lo << 16)) * scale;
             const float c = (__uint_as_float(hi & 0xffff0000u) + __uint_as_float(lo & 0xffff0000u)) * scale;
