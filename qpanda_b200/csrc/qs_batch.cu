@@ -826,38 +826,53 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
     bool want_tmem = o.tile_in_tmem && o.max_sub <= 2;
     std::vector<int> prc(np, QS_OK);
     std::vector<std::string> perr(np);
+    auto pass_blocks = [](const qs_plan *pp, const PlanPass &pass, int (*qpos)[5]) {
+        for (size_t b = 0; b < pass.count; ++b)
+            for (int j = 0; j < 5; ++j) qpos[b][j] = pp->blocks[pass.first + b].q[j];
+    };
     if (!r)
         parallel(np, [&](int pi) {
             const int c = proto_rep[pi];
-            int rr = qs_plan_create_ex(B->nq_eff[c], gates + offsets[c], offsets[c + 1] - offsets[c], &po, &protos[pi]);
+            const int rr = qs_plan_create_ex(B->nq_eff[c], gates + offsets[c], offsets[c + 1] - offsets[c], &po, &protos[pi]);
             const qs_plan *pp = protos[pi];
+            for (size_t u = 0; !rr && want_tmem && u < pp->passes.size() && tl_ok[pi]; ++u) {
+                // the pass for k_batch_tmem: in place, natural layout
+                const PlanPass &pass = pp->passes[u];
+                qs_tiled_desc d;
+                memset(&d, 0, sizeof(d));
+                for (int t = 0; t < 12; ++t) d.T[t] = pass.T[t];
+                d.nsub = (int)pass.count;
+                pass_blocks(pp, pass, d.qpos);
+                qs_tmem::TLayout TL;
+                if (qs_tmem_layout_build(pp->n, &d, &TL) == QS_OK) p_tl[pi].push_back(TL);
+                else tl_ok[pi] = 0;                             // the batch stays on k_batch
+                Layout L;
+                memset(&L, 0, sizeof(L));
+                L.pad = (int32_t)pass.first;                    // all that k_batch_tmem reads of it
+                p_layouts[pi].push_back(L);
+            }
+            if (rr) perr[pi] = qs_last_error();
+            prc[pi] = rr;
+        });
+    for (int pi = 0; pi < np && want_tmem; ++pi) want_tmem = tl_ok[pi] != 0;   // one kernel for the batch
+    if (!r && !want_tmem)
+        parallel(np, [&](int pi) {
+            int rr = prc[pi];
+            const qs_plan *pp = protos[pi];
+            p_layouts[pi].clear();
             for (size_t u = 0; !rr && u < pp->passes.size(); ++u) {
                 const PlanPass &pass = pp->passes[u];
                 Layout L;
                 LoadMap M;
-                int qpos[3][5];
-                for (size_t b = 0; b < pass.count; ++b)
-                    for (int j = 0; j < 5; ++j) qpos[b][j] = pp->blocks[pass.first + b].q[j];
-                int rows[3][7];
+                int qpos[3][5], rows[3][7];
+                pass_blocks(pp, pass, qpos);
                 if ((rr = qs_tile_row_orders(pp->n, pass.T, (int)pass.count, qpos, rows, nullptr, input_mode))) break;
                 if ((rr = qs_tile_layout_build(pp->n, pass.T, (int)pass.count, qpos, rows, &L, &M))) break;
                 L.pad = (int32_t)pass.first;
                 p_layouts[pi].push_back(L);
                 p_loads[pi].push_back(M);
-                if (want_tmem && tl_ok[pi]) {
-                    // the same pass for k_batch_tmem: in place, natural layout
-                    qs_tiled_desc d;
-                    memset(&d, 0, sizeof(d));
-                    for (int t = 0; t < 12; ++t) d.T[t] = pass.T[t];
-                    d.nsub = (int)pass.count;
-                    for (size_t b = 0; b < pass.count; ++b)
-                        for (int j = 0; j < 5; ++j) d.qpos[b][j] = qpos[b][j];
-                    qs_tmem::TLayout TL;
-                    if (qs_tmem_layout_build(pp->n, &d, &TL) == QS_OK) p_tl[pi].push_back(TL);
-                    else tl_ok[pi] = 0;                         // this structure stays on k_batch
-                }
             }
-            if (rr) perr[pi] = qs_last_error();
+            if (rr && !prc[pi]) perr[pi] = qs_last_error();
             prc[pi] = rr;
         });
     for (int pi = 0; pi < np && !r; ++pi)
@@ -875,7 +890,6 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
     std::vector<LoadMap> loads;                       // their tile-order copy maps
     std::vector<qs_tmem::TLayout> tlayouts;           // and tensor-memory layouts (same indices)
     std::vector<size_t> layout_first(np);
-    for (int pi = 0; pi < np && want_tmem; ++pi) want_tmem = tl_ok[pi] != 0;   // one kernel for the batch
     B->use_tmem = want_tmem;
     for (int pi = 0; pi < np && !r; ++pi) {
         layout_first[pi] = layouts.size();
@@ -965,7 +979,7 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
             bc.amp = reinterpret_cast<float *>(static_cast<char *>(B->d_states) + B->amp_off[c]);
             bc.mats = static_cast<const uint16_t *>(B->d_mats) + mat_off[c];
             bc.layouts = static_cast<const Layout *>(B->d_layouts) + layout_first[proto_id[c]];
-            bc.loads = static_cast<const LoadMap *>(B->d_loads) + layout_first[proto_id[c]];
+            bc.loads = want_tmem ? nullptr : static_cast<const LoadMap *>(B->d_loads) + layout_first[proto_id[c]];
             bc.tlayouts = want_tmem ? static_cast<const qs_tmem::TLayout *>(B->d_tlayouts) + layout_first[proto_id[c]]
                                     : nullptr;
             bc.zz = B->d_zz + B->zz_off[c];

@@ -138,77 +138,74 @@ Groups closure_groups(const std::vector<size_t> &idx, const std::vector<uint64_t
 {
     Groups out;
     const size_t N = idx.size();
-    std::vector<char> done(N, 0);
-    size_t left = N, first = 0;
-    // How many gates the closure of Q would take (and which, in *take when
-    // take is non-null), gates marked in `trial` counting as placed: repeated
-    // scans in list order; a scan stops once every qubit of Q is held by an
-    // earlier unplaced non-diagonal gate.
-    std::vector<char> trial(N, 0);
-    auto closure = [&](uint64_t Q, std::vector<size_t> *take) {
+    size_t left = N;
+    // the unplaced gates, in list order
+    struct Gate {
+        uint64_t m;
+        size_t t;
+        bool d, placed;
+    };
+    std::vector<Gate> rest(N);
+    for (size_t t = 0; t < N; ++t) rest[t] = {mask[idx[t]], t, diag[idx[t]] != 0, false};
+    auto compact = [&]() {
+        size_t o = 0;
+        for (const Gate &g : rest)
+            if (!g.placed) rest[o++] = g;
+        rest.resize(o);
+    };
+    // How many gates the closure of Q would take, the gate at `skip` counting
+    // as placed; with mem, takes them.  One scan in list order: what a gate
+    // needs is that no unplaced gate before it fails to commute with it, and
+    // a gate taken later in the scan does not change that.  The scan stops
+    // once every qubit of Q is held by an earlier unplaced non-diagonal gate.
+    auto closure = [&](uint64_t Q, size_t skip, std::vector<size_t> *mem) {
         int n = 0;
-        std::vector<size_t> touched;
-        bool changed = true;
-        while (changed) {
-            changed = false;
-            Blocker bl;
-            for (size_t t = first; t < N && (Q & ~bl.any); ++t) {
-                if (done[t] || trial[t]) continue;
-                const uint64_t m = mask[idx[t]];
-                const bool d = diag[idx[t]];
-                if (bl.free(m, d) && !(m & ~Q)) {
-                    trial[t] = 1;
-                    touched.push_back(t);
-                    ++n;
-                    changed = true;
-                } else {
-                    bl.add(m, d);
+        uint64_t any = 0, dg = 0;
+        const size_t size = rest.size();
+        for (size_t i = 0; i < size && (Q & ~any); ++i) {
+            Gate &g = rest[i];
+            if (g.placed || i == skip) continue;
+            if (!(g.m & any) && (g.d || !(g.m & dg)) && !(g.m & ~Q)) {
+                ++n;
+                if (mem) {
+                    g.placed = true;
+                    mem->push_back(idx[g.t]);
                 }
+            } else {
+                (g.d ? dg : any) |= g.m;
             }
         }
-        for (size_t t : touched) trial[t] = 0;
-        if (take) *take = std::move(touched);
         return n;
-    };
-    auto place = [&](size_t t, uint64_t &Q, std::vector<size_t> &mem) {
-        done[t] = 1;
-        --left;
-        Q |= mask[idx[t]];
-        mem.push_back(idx[t]);
     };
     uint64_t all_q = 0;                      // every qubit the gates touch
     for (size_t t = 0; t < N; ++t) all_q |= mask[idx[t]];
     uint64_t pass_T = tile_low;              // tile so far of the pass being filled (tile_q > 0)
     int in_pass = 0;
     while (left) {
-        while (first < N && done[first]) ++first;
-        if (tile_q > 0 && in_pass > 0 && __builtin_popcountll(pass_T | mask[idx[first]]) > tile_q) {
+        if (tile_q > 0 && in_pass > 0 && __builtin_popcountll(pass_T | rest[0].m) > tile_q) {
             pass_T = tile_low;               // the next gate does not fit this pass: start a new one
             in_pass = 0;
         }
         const uint64_t budget_T = tile_q > 0 && in_pass > 0 ? pass_T : 0;
-        uint64_t Q = 0;
         std::vector<size_t> mem;
-        place(first, Q, mem);                // seed: the first unplaced gate
+        uint64_t Q = rest[0].m;              // seed: the first unplaced gate
+        mem.push_back(idx[rest[0].t]);
+        rest[0].placed = true;
         while (true) {
-            std::vector<size_t> take;
-            closure(Q, &take);
-            for (size_t t : take) place(t, Q, mem);
+            closure(Q, N, &mem);
+            compact();
             Blocker bl;                      // grow: available gates that fit
             int best_n = -1, best_add = 65;
             size_t best = N;
             int evaluated = 0;               // the first kMaxCandidates available gates are tried
-            for (size_t t = first; t < N && (all_q & ~bl.any) && evaluated < kMaxCandidates; ++t) {
-                if (done[t]) continue;
-                const uint64_t m = mask[idx[t]];
-                const bool d = diag[idx[t]];
+            for (size_t i = 0; i < rest.size() && (all_q & ~bl.any) && evaluated < kMaxCandidates; ++i) {
+                const uint64_t m = rest[i].m;
+                const bool d = rest[i].d;
                 if (bl.free(m, d) && __builtin_popcountll(Q | m) <= k &&
                     (!budget_T || __builtin_popcountll(budget_T | Q | m) <= tile_q)) {
                     const int add = __builtin_popcountll(m & ~Q);
                     ++evaluated;
-                    trial[t] = 1;
-                    const int got = closure(Q | m, nullptr);
-                    trial[t] = 0;
+                    const int got = closure(Q | m, i, nullptr);
                     // by ratio: (got + 1) / max(add, 1) against the best's, cross-multiplied
                     const long lhs = (long)(got + 1) * (best_add > 1 ? best_add : 1);
                     const long rhs = (long)(best_n + 1) * (add > 1 ? add : 1);
@@ -217,14 +214,17 @@ Groups closure_groups(const std::vector<size_t> &idx, const std::vector<uint64_t
                     if (better) {
                         best_n = got;
                         best_add = add;
-                        best = t;
+                        best = i;
                     }
                 }
                 bl.add(m, d);
             }
             if (best == N) break;
-            place(best, Q, mem);
+            Q |= rest[best].m;
+            mem.push_back(idx[rest[best].t]);
+            rest[best].placed = true;
         }
+        left -= mem.size();
         if (tile_q > 0) {
             pass_T |= Q;
             if (++in_pass == per_pass) {
@@ -486,11 +486,6 @@ int build_passes(qs_plan *P)
             P->blocks.push_back(std::move(B));
         }
         pass.count = P->blocks.size() - pass.first;
-        int qpos[3][5];
-        for (size_t k = 0; k < pass.count && k < 3; ++k)
-            for (int j = 0; j < 5; ++j) qpos[k][j] = P->blocks[pass.first + k].q[j];
-        if (P->n >= TQ && (r = qs_tile_row_orders(P->n, pass.T, (int)pass.count, qpos, pass.rows)))
-            return r;                        // narrower states run the gates per gate
         P->passes.push_back(pass);
     }
     return QS_OK;
@@ -702,13 +697,9 @@ static void tiled_pass_desc(const qs_plan *P, size_t u, bool last, int mode, std
     d.first_block = pp.first;
     for (size_t b = 0; b < pp.count; ++b)
         for (int j = 0; j < 5; ++j) d.qpos[b][j] = pos[P->blocks[pp.first + b].q[j]];
-    d.has_rows = 1;
     bool ident = true;
     for (int q = 0; q < n; ++q) ident = ident && pos[q] == q;
-    // row orders: the plan's (chosen for the natural layout, written in
-    // place); a permuted layout or write map gets its own at the end
-    for (size_t b = 0; b < pp.count; ++b)
-        for (int i = 0; i < 7; ++i) d.rows[b][i] = pos[pp.rows[b][i]];
+    d.has_rows = 0;                         // tiled_rows
     d.has_write = 0;
     if (last && ident) return;              // natural in, natural out: in place
     d.has_write = 1;
@@ -808,15 +799,23 @@ static void tiled_pass_desc(const qs_plan *P, size_t u, bool last, int mode, std
             if (!((tmask >> p) & 1)) { npos[at[p]] = 12 + i; d.wpos[i] = 12 + i; ++i; }
         d.wmode = 1;
     }
-    // which tile bits are lowest - and so which lanes read and write what -
-    // depends on the positions: choose the row orders for this layout
-    int rows[3][7];
-    if (qs_tile_row_orders(n, d.T, d.nsub, d.qpos, rows, d.wtile, 0) == QS_OK) memcpy(d.rows, rows, sizeof(rows));
     pos.swap(npos);
 }
 
+// The row orders of a pass: which tile bits are lowest - and so which lanes
+// read and write what - depends on its positions and write map.  Only
+// k_fused_tile uses them, and they are most of a pass's host work (0.1 ms, 0.5
+// ms remapped), so k_tile_tmem's passes go without.
+static int tiled_rows(int n, qs_tiled_desc &d)
+{
+    if (d.has_rows) return QS_OK;
+    const int r = qs_tile_row_orders(n, d.T, d.nsub, d.qpos, d.rows, d.has_write ? d.wtile : nullptr, 0);
+    if (!r) d.has_rows = 1;
+    return r;
+}
+
 int qs_plan_tiled_schedule(const qs_plan *P, int n, size_t first, size_t count, int remap,
-                           std::vector<qs_tiled_desc> &descs, std::vector<int> &dst)
+                           std::vector<qs_tiled_desc> &descs, std::vector<int> &dst, bool rows)
 {
     if (P->opts.kernel != QS_PLAN_TILED || n != P->n || first > P->passes.size() ||
         count > P->passes.size() - first)
@@ -843,6 +842,8 @@ int qs_plan_tiled_schedule(const qs_plan *P, int n, size_t first, size_t count, 
             dst[k] = cur ^ 1;
             cur ^= 1;
         }
+        const int r = rows && n >= 12 ? tiled_rows(n, d) : QS_OK;
+        if (r) return r;
     }
     return QS_OK;
 }
@@ -907,7 +908,7 @@ extern "C" int qs_plan_apply_range(qs_state *s, qs_plan *P, size_t first, size_t
         // the plan for its next application over the same range
         if (P->sched_remap != remap || P->sched_first != first || P->sched_count != count) {
             P->sched_remap = -1;
-            if ((r = qs_plan_tiled_schedule(P, s->n, first, count, remap, P->sched, P->sched_dst))) return r;
+            if ((r = qs_plan_tiled_schedule(P, s->n, first, count, remap, P->sched, P->sched_dst, false))) return r;
             P->sched_remap = remap;
             P->sched_first = first;
             P->sched_count = count;
@@ -930,7 +931,13 @@ extern "C" int qs_plan_apply_range(qs_state *s, qs_plan *P, size_t first, size_t
             d.out_parts = norm + GT * (1 + u % 2);
             r = QS_ERR_UNSUPPORTED;
             if (P->opts.tile_in_tmem) r = qs_launch_tiled_tmem(s, &d, flag);
-            if (r == QS_ERR_UNSUPPORTED) r = qs_launch_tiled(s, &d, flag);
+            if (r == QS_ERR_UNSUPPORTED) {
+                qs_tiled_desc &kept = P->sched[u - first];      // computed once, with the schedule
+                if ((r = tiled_rows(s->n, kept))) return r;
+                d.has_rows = 1;
+                memcpy(d.rows, kept.rows, sizeof(d.rows));
+                r = qs_launch_tiled(s, &d, flag);
+            }
             if (r) return r;
         }
         // the rescale of each pass leaves only the last pass's drift

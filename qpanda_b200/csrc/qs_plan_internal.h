@@ -22,7 +22,6 @@ struct PlanBlock {
 struct PlanPass {
     int T[12] = {0};                     // ascending global qubits of the tile
     size_t first = 0, count = 0;         // its blocks: blocks[first, first + count)
-    int rows[3][7] = {};                 // each block's other tile qubits in row-bit order (qs_tile_row_orders)
 };
 
 struct qs_plan {
@@ -59,7 +58,8 @@ struct qs_tiled_desc;
 // the other).  With remap (qs_plan_opts.remap), passes ping-pong through the
 // spare buffer, each writing the layout that makes its own stores (1) or the
 // next pass's loads (2) contiguous tiles, and the last writes the natural
-// order; the state's own buffer holds the result.  Pure host code (also used by the CPU
+// order; the state's own buffer holds the result.  rows: choose each pass's row
+// orders (k_fused_tile's) too.  Pure host code (also used by the CPU
 // emulation test of the tiled passes).
 int qs_plan_tiled_schedule(const qs_plan *P, int n, size_t first, size_t count, int remap,
-                           std::vector<qs_tiled_desc> &descs, std::vector<int> &dst);
+                           std::vector<qs_tiled_desc> &descs, std::vector<int> &dst, bool rows = true);

@@ -455,7 +455,11 @@ struct Planner {
     std::vector<Term> terms;
     std::vector<int> left;       // ops not yet in a pass, in order
 private:
-    int scan(uint64_t q, std::vector<uint64_t> *wants, std::vector<int> *taken) const;
+    struct Masks {
+        uint64_t tgt, diag;
+        int op;
+    };
+    int scan(const std::vector<Masks> &list, uint64_t q, std::vector<uint64_t> *wants, std::vector<Masks> *kept) const;
 };
 
 // The stages of a pass (a RunSmall or RunLarge): fills R from pass_ops on the

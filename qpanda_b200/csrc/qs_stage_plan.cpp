@@ -154,20 +154,22 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
         if (ops[i].type != G_NONE) left.push_back((int)i);
 }
 
-// Ops of `left` that can run in a pass on the tile of q: their targets in q,
-// and they commute with every earlier op that stays behind.  Returns their
-// number; *taken gets them, *wants the target sets that alone keep an op out.
-int Planner::scan(uint64_t q, std::vector<uint64_t> *wants, std::vector<int> *taken) const
+// The ops of list that can run in a pass on the tile of q: their targets in
+// q, and they commute with every earlier op that stays behind.  Returns their
+// number; *wants gets the target sets that alone keep an op out, *kept the
+// ops that stay behind (the rest of the list from where nothing can run).
+int Planner::scan(const std::vector<Masks> &list, uint64_t q, std::vector<uint64_t> *wants,
+                  std::vector<Masks> *kept) const
 {
     const uint64_t all = n >= 64 ? ~0ull : (1ull << n) - 1;
     uint64_t skip_all = 0, skip_tgt = 0;
     int count = 0;
-    for (int i : left) {
-        const GOp &g = ops[(size_t)i];
+    const size_t size = list.size();
+    for (size_t i = 0; i < size; ++i) {
+        const Masks &g = list[i];
         const bool free = !(g.tgt & skip_all) && !(g.diag & skip_tgt);
         if (free && !(g.tgt & ~q)) {
             ++count;
-            if (taken) taken->push_back(i);
             continue;
         }
         if (free && wants) {
@@ -176,7 +178,11 @@ int Planner::scan(uint64_t q, std::vector<uint64_t> *wants, std::vector<int> *ta
         }
         skip_all |= g.tgt | g.diag;
         skip_tgt |= g.tgt;
-        if ((skip_tgt & all) == all) break;
+        if (kept) kept->push_back(g);
+        if ((skip_all & all) == all) {
+            if (kept) kept->insert(kept->end(), list.begin() + (long)i + 1, list.end());
+            break;
+        }
     }
     return count;
 }
@@ -186,37 +192,52 @@ bool Planner::next(uint64_t *qmask, std::vector<int> *pass_ops)
     pass_ops->clear();
     if (left.empty()) return false;
     uint64_t q = n <= K ? (1ull << n) - 1 : (1ull << low) - 1;
-    if (n > K) {
-        // grow the tile by the target set that lets the most ops per qubit in
-        int have = scan(q, nullptr, nullptr);
-        std::vector<uint64_t> wants;
-        while (popc(q) < K) {
-            wants.clear();
-            scan(q, &wants, nullptr);
-            uint64_t best = 0;
-            double best_gain = -1;
-            int best_count = 0;
-            for (uint64_t w : wants) {
-                const int c = scan(q | w, nullptr, nullptr);
-                const double gain = (double)(c - have) / popc(w);
-                if (gain > best_gain) {
-                    best_gain = gain;
-                    best = w;
-                    best_count = c;
-                }
+    // the ops that stay behind so far: what runs on a tile runs on every
+    // larger one, so a round looks at the rest only
+    std::vector<Masks> rest, behind;
+    rest.reserve(left.size());
+    for (int i : left) rest.push_back({ops[(size_t)i].tgt, ops[(size_t)i].diag, i});
+    behind.reserve(left.size());
+    std::vector<uint64_t> wants;
+    double last[64];                               // a qubit's gain when it was last looked at
+    for (double &g : last) g = 1e9;
+    while (true) {
+        wants.clear();
+        behind.clear();
+        scan(rest, q, popc(q) < K ? &wants : nullptr, &behind);
+        rest.swap(behind);
+        if (popc(q) >= K) break;
+        // grow the tile by the target set that lets the most ops per qubit in;
+        // gains change little from round to round, so sets are looked at by
+        // their last gain, and not those whose last gain is below half the best
+        auto guess = [&](uint64_t w) { return popc(w) == 1 ? last[low_bit(w)] : 1e8; };
+        std::stable_sort(wants.begin(), wants.end(), [&](uint64_t x, uint64_t y) { return guess(x) > guess(y); });
+        uint64_t best = 0;
+        double best_gain = -1;
+        for (uint64_t w : wants) {
+            if (guess(w) < best_gain * 0.5) break;
+            const double gain = (double)scan(rest, q | w, nullptr, nullptr) / popc(w);
+            if (popc(w) == 1) last[low_bit(w)] = gain;
+            if (gain > best_gain) {
+                best_gain = gain;
+                best = w;
             }
-            if (!best) break;
+        }
+        if (best) {
             q |= best;
-            have = best_count;
+            continue;
         }
         for (int b = 0; b < n && popc(q) < K; ++b) q |= 1ull << b;
     }
-    scan(q, nullptr, pass_ops);
-    // left minus pass_ops (both ascending)
+    // the pass: what did not stay behind (both ascending)
     size_t k = 0, o = 0;
     for (size_t i = 0; i < left.size(); ++i) {
-        if (k < pass_ops->size() && left[i] == (*pass_ops)[k]) { ++k; continue; }
-        left[o++] = left[i];
+        if (k < rest.size() && left[i] == rest[k].op) {
+            ++k;
+            left[o++] = left[i];
+        } else {
+            pass_ops->push_back(left[i]);
+        }
     }
     left.resize(o);
     *qmask = q;
@@ -324,31 +345,49 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         for (qs &= qmask; qs; qs &= qs - 1) o |= 1u << ps[low_bit(qs)];
         return o;
     };
-    std::vector<int> todo(pass_ops), take;
-    // ops of todo that run in a stage with these register bits (tile bits)
-    auto scan = [&](uint32_t regs, std::vector<uint32_t> *wants, std::vector<int> *taken) {
-        uint64_t skip_all = 0, skip_tgt = 0;
-        int count = 0, ps[64];
-        bool moved = false;
-        const int *cur = pos;
-        for (int i : todo) {
-            const GOp &g = P.ops[(size_t)i];
-            const bool free = !(g.tgt & skip_all) && !(g.diag & skip_tgt);
-            if (free) {
-                if (g.type == G_SWAP) {
-                    if (!moved) {
-                        memcpy(ps, pos, sizeof(ps));
-                        cur = ps;
-                        moved = true;
-                    }
-                    std::swap(ps[low_bit(g.off0)], ps[low_bit(g.off1)]);
-                    if (taken) taken->push_back(i);
+    // The pass's ops with their qubits as tile bits at the load: which ops may
+    // pass which does not depend on where a SWAP has put a qubit since.
+    struct Todo {
+        uint32_t tgt, diag;
+        int op;
+        bool swap;
+    };
+    int home[64];
+    memcpy(home, pos, sizeof(home));
+    std::vector<Todo> todo;
+    std::vector<int> take;
+    bool swaps = false;
+    todo.reserve(pass_ops.size());
+    for (int i : pass_ops) {
+        const GOp &g = P.ops[(size_t)i];
+        todo.push_back({tile_bits(g.tgt, pos), tile_bits(g.diag, pos), i, g.type == G_SWAP});
+        swaps = swaps || g.type == G_SWAP;
+    }
+    int at[kMaxTile];                              // tile bit of a qubit now, by its tile bit at the load
+    for (int b = 0; b < K; ++b) at[b] = b;
+    // ops of list that run in a stage with these register bits (tile bits now)
+    auto scan = [&](const std::vector<Todo> &list, uint32_t regs, std::vector<uint32_t> *wants,
+                    std::vector<int> *taken, std::vector<Todo> *kept) {
+        const uint32_t all = (1u << K) - 1;
+        uint32_t skip_all = 0, skip_tgt = 0;
+        int count = 0, ps[kMaxTile];
+        if (swaps) memcpy(ps, at, sizeof(ps));
+        for (size_t i = 0; i < list.size(); ++i) {
+            const Todo &g = list[i];
+            if (!(g.tgt & skip_all) && !(g.diag & skip_tgt)) {
+                if (g.swap) {
+                    std::swap(ps[low_bit(g.tgt)], ps[31 - __builtin_clz(g.tgt)]);
+                    if (taken) taken->push_back(g.op);
                     continue;
                 }
-                const uint32_t t = tile_bits(g.tgt, cur);
+                uint32_t t = g.tgt;
+                if (swaps) {
+                    t = 0;
+                    for (uint32_t m = g.tgt; m; m &= m - 1) t |= 1u << ps[low_bit(m)];
+                }
                 if (!(t & ~regs)) {
-                    count += g.tgt ? 2 : 0;        // what needs no register bit runs in any stage
-                    if (taken) taken->push_back(i);
+                    count += t ? 1 : 0;            // what needs no register bit runs in any stage
+                    if (taken) taken->push_back(g.op);
                     continue;
                 }
                 const uint32_t w = t & ~regs;
@@ -357,7 +396,11 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
             }
             skip_all |= g.tgt | g.diag;
             skip_tgt |= g.tgt;
-            if ((skip_tgt & qmask) == qmask) break;
+            if (kept) kept->push_back(g);
+            if (skip_all == all) {
+                if (kept) kept->insert(kept->end(), list.begin() + (long)i + 1, list.end());
+                break;
+            }
         }
         return count;
     };
@@ -365,25 +408,31 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
     double growth = 1;
     int nops = 0, nent = 0;
     const uint32_t low_tile = (1u << LOW) - 1, all_tile = (1u << K) - 1;
+    std::vector<Todo> rest_of, behind;
+    std::vector<uint32_t> wants;
     auto choose = [&](uint32_t allowed) {
         uint32_t regs = 0;
-        std::vector<uint32_t> wants;
-        int have = scan(0, nullptr, nullptr);
+        rest_of = todo;
         while (popc(regs) < RB) {
             wants.clear();
-            scan(regs, &wants, nullptr);
+            if (swaps) {
+                scan(todo, regs, &wants, nullptr, nullptr);
+            } else {                               // as in next(): a round looks at what stays behind only
+                behind.clear();
+                scan(rest_of, regs, &wants, nullptr, &behind);
+                rest_of.swap(behind);
+            }
+            const int have = swaps ? scan(todo, regs, nullptr, nullptr, nullptr) : 0;
             uint32_t best = 0;
             double best_gain = -1;
-            int best_count = 0;
             for (uint32_t w : wants) {
                 if (w & ~allowed) continue;
-                const int c = scan(regs | w, nullptr, nullptr);
-                const double gain = (double)(c - have) / popc(w);
-                if (gain > best_gain) { best_gain = gain; best = w; best_count = c; }
+                const double gain =
+                    (double)(scan(swaps ? todo : rest_of, regs | w, nullptr, nullptr, nullptr) - have) / popc(w);
+                if (gain > best_gain) { best_gain = gain; best = w; }
             }
             if (!best) break;
             regs |= best;
-            have = best_count;
         }
         for (int b = K - 1; b >= 0 && popc(regs) < RB; --b)
             if (allowed >> b & 1) regs |= 1u << b;
@@ -446,6 +495,8 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
     // one op at the current stage; false when it does not fit the parameter block
     auto emit = [&](const GOp &g) {
         if (g.type == G_SWAP) {
+            const uint32_t t = tile_bits(g.tgt, home);
+            std::swap(at[low_bit(t)], at[31 - __builtin_clz(t)]);
             std::swap(pos[low_bit(g.off0)], pos[low_bit(g.off1)]);
             return true;
         }
@@ -521,7 +572,7 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         const bool first = S.nstages == 0;
         const uint32_t regs = choose(first ? all_tile & ~low_tile : all_tile);
         take.clear();
-        scan(regs, nullptr, &take);
+        scan(todo, regs, nullptr, &take, nullptr);
         // the store reads the tile with the lowest qubits on the lowest lanes
         int ps[64], lanes[LOW];
         memcpy(ps, pos, sizeof(ps));
@@ -549,12 +600,12 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         st->count = (uint16_t)(nops - st->first);
         // todo minus what was emitted
         for (size_t i = 0, e = 0; i < todo.size(); ++i) {
-            if (e < k && todo[i] == take[e]) { ++e; continue; }
+            if (e < k && todo[i].op == take[e]) { ++e; continue; }
             todo[t++] = todo[i];
         }
         todo.resize(t);
         if (full || S.nstages + 1 >= R::NST) {
-            *rest = todo;
+            for (const Todo &o : todo) rest->push_back(o.op);
             todo.clear();
             full = true;
         }
@@ -572,15 +623,15 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         }
     }
     // state offsets of the load (first stage) and the store (last stage)
-    int at[kMaxTile];                              // qubit behind a tile bit at the store
+    int stored_q[kMaxTile];                        // qubit behind a tile bit at the store
     for (int q = 0; q < n; ++q)
-        if (pos[q] >= 0) at[pos[q]] = q;
+        if (pos[q] >= 0) stored_q[pos[q]] = q;
     auto offsets = [&](const Stage &st, const int *regs, const int *qs, uint32_t *gt, uint32_t *gr) {
         for (int j = LOW; j < tbits; ++j) gt[j] = 1u << (qs[low_bit(st.tb[j] & 0xffffu)] - LOW);
         for (int j = 0; j < RB; ++j) gr[j] = 1u << (qs[regs[j]] - LOW);
     };
     offsets(S.st[0], reg_in, qubit, S.gin_t, S.gin_r);
-    offsets(S.st[S.nstages - 1], reg_at, at, S.gout_t, S.gout_r);
+    offsets(S.st[S.nstages - 1], reg_at, stored_q, S.gout_t, S.gout_r);
     S.scale[0] = (T)scale.real();
     S.scale[1] = (T)scale.imag();
     S.scale_kind = scale.imag() != 0 ? 2 : scale.real() != 1 ? 1 : 0;
