@@ -176,7 +176,7 @@ struct MargParams {
     int ulo_pos[12];
     int mhi_pos[40], mhi_out[40];
     int uhi_pos[40];
-    uint64_t G, R;               // slices of the unmeasured high space, chunks per CTA
+    uint64_t G, R, uspace;       // slices of the unmeasured high space, chunks per slice (at most), chunks
 };
 
 template <typename T>
@@ -278,13 +278,15 @@ k_marginal(const T *__restrict__ a, MargParams P, double *__restrict__ part)
 // The same marginal on chunks of 4096 (states of 12 qubits and more): a
 // thread owns fixed chunk positions and adds their |a|^2 in registers, chunk
 // after chunk, with 16-byte loads (two complex64 or one complex128 amplitude
-// each) and two chunks' loads in flight before their first use.  When every
+// each), the next loads in flight while the last ones are added.  When every
 // chunk bit is measured (P.ulo == 0) each position is a bin - the order
 // k_marginal adds them in, so the bins are bit-identical - and no shared
 // memory is used; otherwise the CTA folds its 4096 position sums into the
 // 2^mlo bins once, at the end, in a fixed order.
-template <typename T, bool FOLD>
-__global__ void __launch_bounds__(kThreads)
+constexpr int kMargCtas = 2;             // resident CTAs per SM of the kernel that streams chunks
+
+template <typename T, bool FOLD, bool ONE>
+__global__ void __launch_bounds__(kThreads, ONE ? 3 : kMargCtas)
 k_marginal_direct(const T *__restrict__ a, MargParams P, double *__restrict__ part)
 {
     constexpr int kApl = sizeof(T) == 4 ? 2 : 1;            // amplitudes per 16-byte load
@@ -308,36 +310,51 @@ k_marginal_direct(const T *__restrict__ a, MargParams P, double *__restrict__ pa
         for (int j = 0; j < P.uhi; ++j) hu |= ((uidx >> j) & 1ull) << P.uhi_pos[j];
         return ((hm | hu) << 12) / kApl;                       // in 16-byte units
     };
-    auto add = [&](const L16 (&v)[kLoads]) {
+    auto add = [&](const L16 (&v)[8], int first) {
 #pragma unroll
-        for (int i = 0; i < kLoads; ++i) {
+        for (int i = 0; i < 8; ++i) {
             if constexpr (sizeof(T) == 4) {
                 const float4 x = *reinterpret_cast<const float4 *>(&v[i]);
-                acc[2 * i] += p2(x.x, x.y);
-                acc[2 * i + 1] += p2(x.z, x.w);
+                acc[2 * (first + i)] += p2(x.x, x.y);
+                acc[2 * (first + i) + 1] += p2(x.z, x.w);
             } else {
                 const double2 x = *reinterpret_cast<const double2 *>(&v[i]);
-                acc[i] += p2(x.x, x.y);
+                acc[first + i] += p2(x.x, x.y);
             }
         }
     };
-    uint64_t r = 0;
-    for (; r + 2 <= P.R; r += 2) {
-        const uint64_t b0 = chunk_base(r), b1 = chunk_base(r + 1);
-        L16 v0[kLoads], v1[kLoads];
+    // A part: 8 loads a thread, a complex64 chunk or half a complex128 one.  One
+    // part's loads stay in flight while another's sums are taken; a CTA of one
+    // chunk (ONE) has nothing to overlap and runs three to an SM instead of
+    // two.  27 qubits complex64 (164 us at the copy's rate): 12 low qubits 351
+    // -> 185 us, 16 spread ones 250 -> 185, the outer two 280 -> 179; 22 qubits,
+    // 12 low ones 117 -> 21 us (their slices were added by a thread per bin).
+    constexpr int kPart = 8, kParts = kLoads / kPart;
+    const uint64_t chunks = g * P.R < P.uspace ? (P.uspace - g * P.R < P.R ? P.uspace - g * P.R : P.R) : 0;
+    auto load = [&](L16 (&v)[kPart], uint64_t r, int h) {
+        const L16 *p = pa + chunk_base(r) + t + h * kPart * kThreads;
 #pragma unroll
-        for (int i = 0; i < kLoads; ++i) v0[i] = __ldg(pa + b0 + t + i * kThreads);
+        for (int i = 0; i < kPart; ++i) v[i] = __ldg(p + i * kThreads);
+    };
+    if constexpr (ONE) {
+        L16 v[kPart];
 #pragma unroll
-        for (int i = 0; i < kLoads; ++i) v1[i] = __ldg(pa + b1 + t + i * kThreads);
-        add(v0);
-        add(v1);
-    }
-    if (r < P.R) {
-        const uint64_t b0 = chunk_base(r);
-        L16 v0[kLoads];
+        for (int h = 0; h < kParts; ++h)
+            if (chunks) {
+                load(v, 0, h);
+                add(v, h * kPart);
+            }
+    } else {
+        L16 v[2][kPart];
+        if (chunks) load(v[0], 0, 0);
+        for (uint64_t r = 0; r < chunks; r += 2 / kParts) {
 #pragma unroll
-        for (int i = 0; i < kLoads; ++i) v0[i] = __ldg(pa + b0 + t + i * kThreads);
-        add(v0);
+            for (int k = 0; k < 2; ++k) {             // two parts: two chunks, or one chunk's halves
+                const uint64_t rn = r + (k + 1) / kParts;
+                if (rn < chunks) load(v[(k + 1) & 1], rn, (k + 1) % kParts);
+                if (kParts == 2 || r + k < chunks) add(v[k], kParts == 2 ? k * kPart : 0);
+            }
+        }
     }
     double *dst = part + g * (1ull << P.m);
     if constexpr (!FOLD) {                                    // every chunk position is a bin
@@ -398,6 +415,19 @@ __global__ void k_marginal_combine(const double *__restrict__ part, uint64_t G, 
         for (uint64_t g = 0; g < G; ++g) s += part[g * nout + o];
         out[o] = s;
     }
+}
+
+// The same with a warp per bin, where the bins are too few to fill the device
+// and the slices many (444 slices of 4 bins: 27 us with a thread per bin).
+__global__ void __launch_bounds__(kThreads)
+k_marginal_combine_warp(const double *__restrict__ part, uint64_t G, uint64_t nout, double *__restrict__ out)
+{
+    const uint64_t o = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
+    if (o >= nout) return;
+    double s = 0;
+    for (uint64_t g = threadIdx.x & 31; g < G; g += 32) s += part[g * nout + o];
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) out[o] = s;
 }
 
 size_t marginal_smem(const MargParams &P)
@@ -697,10 +727,30 @@ MargParams marginal_plan(const qs_state *s, const int *qubits, int m, size_t *pa
     }
     // Aim for ~4 CTAs per SM in total.
     uint64_t ohi = 1ull << P.mhi, uspace = 1ull << P.uhi;
+    P.uspace = uspace;
     uint64_t G = 1;
-    while (G < uspace && ohi * G < (uint64_t)QS_SM_COUNT * 4) G <<= 1;
+    if (P.c < 12) {
+        while (G < uspace && ohi * G < (uint64_t)QS_SM_COUNT * 4) G <<= 1;
+    } else {
+        // Slices are cut so that the CTAs of k_marginal_direct come out at whole
+        // waves (as a power of two they came to 2.3 of 3, or 1.2 of 2).  Time of w
+        // waves: their chunks at HBM rate, plus the slices' partials written,
+        // read and added (in bytes per CTA slot, both sides at the same rate).
+        const uint64_t slots = (uint64_t)QS_SM_COUNT * kMargCtas;
+        const double chunk = 4096.0 * (s->dtype == QS_C64 ? 8 : 16) * (double)slots;
+        double best = -1;
+        for (uint64_t w = 1; w <= 8; ++w) {
+            const uint64_t g = std::min(uspace, std::max<uint64_t>(1, slots * w / ohi));
+            const uint64_t waves = (ohi * g + slots - 1) / slots;
+            const double t = (double)(waves * ((uspace + g - 1) / g)) * chunk + (g > 1 ? (2.0 * (double)g + 1) * (8ull << m) : 0);
+            if (best < 0 || t < best) {
+                best = t;
+                G = g;
+            }
+        }
+    }
     P.G = G;
-    P.R = uspace / G;
+    P.R = (uspace + G - 1) / G;
     *part_bytes = G > 1 ? G * (8ull << m) : 0;
     return P;
 }
@@ -718,11 +768,10 @@ int marginal_launch(qs_state *s, const MargParams &P, double *dev_out, double *p
     if (P.c == 12) {
         // chunk positions accumulated in registers; folded into bins at the end
         // when some chunk bits are unmeasured (4096 + kThreads doubles of shared memory)
-        if (P.ulo == 0)
-            k_marginal_direct<T, false><<<(unsigned)ctas, kThreads, 0, s->stream>>>(static_cast<const T *>(s->amp), P, part);
-        else
-            k_marginal_direct<T, true><<<(unsigned)ctas, kThreads, (4096 + kThreads) * sizeof(double), s->stream>>>(
-                static_cast<const T *>(s->amp), P, part);
+        const size_t fold = P.ulo ? (4096 + kThreads) * sizeof(double) : 0;
+        const auto kernel = P.ulo ? (P.R == 1 ? k_marginal_direct<T, true, true> : k_marginal_direct<T, true, false>)
+                                  : (P.R == 1 ? k_marginal_direct<T, false, true> : k_marginal_direct<T, false, false>);
+        kernel<<<(unsigned)ctas, kThreads, fold, s->stream>>>(static_cast<const T *>(s->amp), P, part);
         QS_LAUNCH_CHECK("k_marginal_direct");
     } else {
         size_t smem = marginal_smem(P);
@@ -732,7 +781,10 @@ int marginal_launch(qs_state *s, const MargParams &P, double *dev_out, double *p
     }
     if (G > 1) {
         uint64_t nout = 1ull << P.m;
-        k_marginal_combine<<<grid_for(nout, kThreads), kThreads, 0, s->stream>>>(part, G, nout, dev_out);
+        if (G >= 32)
+            k_marginal_combine_warp<<<(unsigned)((nout * 32 + kThreads - 1) / kThreads), kThreads, 0, s->stream>>>(part, G, nout, dev_out);
+        else
+            k_marginal_combine<<<grid_for(nout, kThreads), kThreads, 0, s->stream>>>(part, G, nout, dev_out);
         QS_LAUNCH_CHECK("k_marginal_combine");
     }
     return QS_OK;
