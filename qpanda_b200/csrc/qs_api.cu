@@ -208,6 +208,7 @@ extern "C" int qs_set_state(qs_state *s, const void *host, int host_dtype)
     if (r) return r;
     if (!host) return qs_fail(QS_ERR_ARG, "qs_set_state: null buffer");
     if (host_dtype != QS_C64 && host_dtype != QS_C128) return qs_fail(QS_ERR_ARG, "qs_set_state: bad dtype");
+    s->untouched = 0;
     return qs_copy_in(s, host, host_dtype);
 }
 

@@ -58,6 +58,11 @@ struct qs_state {
     // Stream-ordered memory (qs_create_async): cudaMallocAsync / cudaFreeAsync
     // on `stream`, and an ordinary host buffer instead of pinned memory.
     bool stream_alloc = false;
+    // Qubits that no gate has mixed since the state was |0...0>: where one of
+    // them is set the amplitudes are zero.  A hint only (the caller can write to
+    // the amplitudes): staged passes that have it look before they leave a
+    // tile alone.
+    uint64_t untouched = 0;
     size_t amp_bytes() const { return N * (dtype == QS_C64 ? 8ull : 16ull); }
 };
 

@@ -267,12 +267,14 @@ int do_phase(qs_state *s, uint64_t mask, double re, double im)
 int launch_pair(qs_state *s, uint64_t holes_mask, uint64_t cmask, uint64_t off0, uint64_t off1,
                 const double m[8])
 {
+    s->untouched &= ~(off0 | off1);
     return s->dtype == QS_C64 ? do_pair<float>(s, holes_mask, cmask, off0, off1, m)
                               : do_pair<double>(s, holes_mask, cmask, off0, off1, m);
 }
 
 int launch_quad(qs_state *s, int q0, int q1, uint64_t cmask, const double m[32])
 {
+    s->untouched &= ~(1ull << q0 | 1ull << q1);
     return s->dtype == QS_C64 ? do_quad<float>(s, q0, q1, cmask, m)
                               : do_quad<double>(s, q0, q1, cmask, m);
 }
@@ -286,6 +288,7 @@ int launch_phase(qs_state *s, uint64_t mask, double re, double im)
 int launch_fill_zero_state(qs_state *s)
 {
     uint64_t nvec = s->amp_bytes() / 16;
+    s->untouched = s->N - 1;
     if (s->dtype == QS_C64)
         k_zero_state<float><<<grid_for(nvec, 256), 256, 0, s->stream>>>(static_cast<float *>(s->amp), nvec);
     else

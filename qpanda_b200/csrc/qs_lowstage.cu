@@ -335,5 +335,6 @@ int qs_launch_lowstage(qs_state *s, const std::vector<qs_prim> &run, uint64_t qm
     for (const qs_prim &p : run)
         if (prim_targets(p) & ~qmask) return qs_fail(QS_ERR_ARG, "staged run: a gate's targets are not tile qubits");
     const TileMap M = {K, qmask};
+    s->untouched = 0;
     return s->dtype == QS_C64 ? launch_run<float>(s, run, M) : launch_run<double>(s, run, M);
 }

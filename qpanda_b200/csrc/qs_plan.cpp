@@ -880,6 +880,7 @@ extern "C" int qs_plan_apply_range(qs_state *s, qs_plan *P, size_t first, size_t
     }
     if (first > plan_launches(P) || count > plan_launches(P) - first)
         return qs_fail(QS_ERR_ARG, "qs_plan_apply_range: launches [%zu, +%zu) out of range", first, count);
+    s->untouched = 0;
     if ((r = qs_plan_upload(P, s))) return r;
     // Norm partials live in their own per-state buffer, so that other calls
     // between two qs_plan_apply_range calls cannot overwrite them:

@@ -42,6 +42,15 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
             v.i[r] = x.y;
         }
     }
+    // The first passes after |0...0> meet tiles of zeros only (a qubit outside
+    // the tile is still in |0> and set in the tile's base).  Gates are linear:
+    // such a tile stays as it is, neither computed nor stored.
+    if (P.zeros) {
+        bool any = false;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) any = any || !(v.r[r] == 0) || !(v.i[r] == 0);
+        if (!__syncthreads_or(any)) return;
+    }
     // the ladders' factors, while the loads are in flight
     V *lane_f = tile + tile_slots<T>(P.K), *warp_f = lane_f + 32 * P.nladders;
     const uint32_t lw = P.K - RB - 5;                          // log2 of the CTA's warps
@@ -185,11 +194,15 @@ int apply_t(qs_state *s, const std::vector<qs_prim> &prims)
     std::vector<int> pass, rest;
     RunSmall<T> small;
     static thread_local RunLarge<T> large;
+    bool finite = true;                          // zero times infinity would not stay zero
+    for (const qs_prim &p : prims)
+        for (int k = 0; s->untouched && k < 8; ++k) finite = finite && std::isfinite(p.m[k]);
     while (P.next(&qmask, &pass)) {
         // a pass that would move more than its gates one by one stays with them
         double traffic = 0;
         for (int i : pass) traffic += op_traffic(P, P.ops[(size_t)i]);
         int r = QS_OK;
+        const bool zeros = finite && (s->untouched & ~qmask) != 0;
         if (pass.size() == 1 || (traffic <= 1.0 && s->amp_bytes() >= (64ull << 20))) {
             for (size_t k = 0; !r && k < pass.size(); ++k) r = launch_op(s, P, P.ops[(size_t)pass[k]]);
             if (r) return r;
@@ -199,13 +212,16 @@ int apply_t(qs_state *s, const std::vector<qs_prim> &prims)
         if ((int)pass.size() < RunSmall<T>::NOP - 1) {
             plan_pass<RunSmall<T>, T>(P, qmask, pass, &small, &rest);
             done = rest.empty();
+            small.zeros = zeros;
             if (done) r = launch<T>(s, small);
         }
         if (!done) {
             plan_pass<RunLarge<T>, T>(P, qmask, pass, &large, &rest);
             if (!rest.empty()) P.give_back(rest);
+            large.zeros = zeros;
             r = launch<T>(s, large);
         }
+        for (int i : pass) s->untouched &= ~P.ops[(size_t)i].tgt;
         if (r) return r;
     }
     return QS_OK;

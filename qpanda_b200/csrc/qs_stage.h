@@ -128,7 +128,7 @@ struct Run {
     int32_t K, nstages, nladders, nseg;
     T scale[2];                            // applied at the store
     int32_t scale_kind;                    // 0: none, 1: real, 2: complex
-    int32_t pad;
+    int32_t zeros;                         // tiles of zeros are likely: they stay as they are
     uint64_t seg_mask[kMaxSeg];            // the tile index's bits, segment by segment ...
     // state offsets, in units of 2^LOW amplitudes, of the load's and the store's
     // thread bits from LOW up (the first LOW are qubits 0..LOW-1) and register bits

@@ -310,7 +310,7 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
     R &S = *out;
     S.K = K;
     S.nstages = S.nladders = 0;
-    S.pad = 0;
+    S.zeros = 0;
     memset(S.gin_t, 0, sizeof(S.gin_t));
     memset(S.gin_r, 0, sizeof(S.gin_r));
     memset(S.gout_t, 0, sizeof(S.gout_t));

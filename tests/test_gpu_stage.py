@@ -1,11 +1,14 @@
 """The staged passes (k_stage) against the oracle: the narrowest states they
 take, one tile, the first states of several tiles, parameter blocks of both
 sizes, and lists that stay on the per-gate kernels."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from oracle.pyoracle import OracleState
 from qpanda_b200 import StateVector, circuits
+from qpanda_b200.capi import check, lib
 from tests.test_stage_emulation import LISTS
 
 pytestmark = pytest.mark.gpu
@@ -44,6 +47,37 @@ def test_wide_states(need_gpu, dtype):
         init = random_state(n, n)
         with StateVector(n, dtype) as sv:
             sv.set_state(init.astype(np.complex64) if dtype == "c64" else init)
+            sv.apply(gates)
+            got = sv.get_state()
+        o = OracleState(n)
+        o.set_state(init)
+        o.apply(gates)
+        assert np.abs(got - o.state()).max() < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("n", [12, 13, 16])
+def test_lists_from_zero_state(need_gpu, n, dtype):
+    """From |0...0> the first passes leave tiles of zeros alone; amplitudes that
+    the caller has put into the state since, through its device address, are
+    no zeros and take part."""
+    import torch
+
+    gates = circuits.random_layers(n, 3, n, iswap_frac=0.2)
+    for put in (False, True):
+        with StateVector(n, dtype) as sv:
+            sv.apply(circuits.random_layers(n, 1, 1))
+            sv.reset()
+            init = np.zeros(1 << n, complex)
+            init[0] = 1
+            if put:
+                p = C.c_void_p()
+                check(lib().qs_device_ptr(sv.handle, C.byref(p)))
+                mem = type("Mem", (), {"__cuda_array_interface__": {
+                    "shape": (1 << n,), "typestr": "<c8" if dtype == "c64" else "<c16", "data": (p.value, False),
+                    "version": 2}})()
+                torch.as_tensor(mem, device="cuda")[(1 << n) - 3] = 0.5
+                init[-3] = 0.5
             sv.apply(gates)
             got = sv.get_state()
         o = OracleState(n)
