@@ -377,6 +377,18 @@ __device__ __forceinline__ double sum_parts(const double *v, int stride, int n)
     return s;
 }
 
+// A pass whose tiles may hold zeros only (Layout::pad): a qubit outside its
+// tile is still in |0>.  The first two or three passes of every circuit.
+constexpr int32_t kZeros = 1 << 30;
+
+__device__ __forceinline__ bool all_zero(const float (&y)[64])
+{
+    bool zero = true;
+#pragma unroll
+    for (int e = 0; e < 64; ++e) zero = zero && y[e] == 0.f;
+    return zero;
+}
+
 // Wait until `need` parts of a circuit are done; false when that took longer
 // than any task can (2 s) or another CTA has failed.
 __device__ bool wait_parts(const int32_t *done, int32_t need, const int *err)
@@ -453,7 +465,9 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
             }
             __syncthreads();
             D::BWords<kTmThreads, 2> words;
-            D::fetch_b(words, C.mats + (size_t)C.layouts[p].pad * 2 * 64 * 64, L);
+            const int32_t first_block = C.layouts[p].pad;
+            const bool zeros = first_block & kZeros;
+            D::fetch_b(words, C.mats + (size_t)(first_block & ~kZeros) * 2 * 64 * 64, L);
             if (shared && p > 0) {
                 // the parts of the previous pass, and their norm
                 if (__syncthreads_or(tid == 0 && !wait_parts(C.done, p * C.nparts, P.err))) { failed = true; break; }
@@ -516,6 +530,20 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                             asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];"
                                          : "=f"(y[2 * j]), "=f"(y[2 * j + 1]) : "r"(stage + ((xrow ^ L.s_col[j]) << 3)));
                     }
+                }
+                if (zeros && !__syncthreads_or(!all_zero(y))) {
+                    // a tile of zeros: written by the first pass, left alone by
+                    // the others (every gather is done: the next copies may go)
+                    if (p == 0) {
+                        const uint64_t obase = tbase | orow;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            *reinterpret_cast<float2 *>(C.amp + 2 * (obase | L.o_col[j])) = make_float2(0.f, 0.f);
+                    } else if (tile + 1 < tiles) {
+                        D::copy_tile<1>(C.amp, tnext, L, stage, g_t, cs_t);
+                    }
+                    tbase = tnext;
+                    continue;
                 }
                 D::split_store<1>(tlane, y, 0u);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -835,6 +863,7 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
             const int c = proto_rep[pi];
             const int rr = qs_plan_create_ex(B->nq_eff[c], gates + offsets[c], offsets[c + 1] - offsets[c], &po, &protos[pi]);
             const qs_plan *pp = protos[pi];
+            uint64_t untouched = (1ull << B->nq_eff[c]) - 1;    // qubits still in |0>
             for (size_t u = 0; !rr && want_tmem && u < pp->passes.size() && tl_ok[pi]; ++u) {
                 // the pass for k_batch_tmem: in place, natural layout
                 const PlanPass &pass = pp->passes[u];
@@ -849,6 +878,8 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
                 Layout L;
                 memset(&L, 0, sizeof(L));
                 L.pad = (int32_t)pass.first;                    // all that k_batch_tmem reads of it
+                for (int t = 0; t < 12; ++t) untouched &= ~(1ull << pass.T[t]);
+                if (untouched) L.pad |= kZeros;
                 p_layouts[pi].push_back(L);
             }
             if (rr) perr[pi] = qs_last_error();
