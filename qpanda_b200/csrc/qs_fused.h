@@ -57,6 +57,7 @@ struct qs_tiled_desc {
     const void *amp_in;
     void *amp_out;
     size_t first_block;          // the plan's index of block 0 of the pass (host bookkeeping)
+    int zeros;                   // tiles of zeros are likely (k_tile_tmem looks and passes them by)
     int threads_per_row;         // 1: 128 threads per lane, a row each; 2: 256, half a row each
 };
 

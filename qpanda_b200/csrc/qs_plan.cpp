@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <complex>
 #include <cstring>
 #include <vector>
@@ -880,6 +881,9 @@ extern "C" int qs_plan_apply_range(qs_state *s, qs_plan *P, size_t first, size_t
     }
     if (first > plan_launches(P) || count > plan_launches(P) - first)
         return qs_fail(QS_ERR_ARG, "qs_plan_apply_range: launches [%zu, +%zu) out of range", first, count);
+    uint64_t untouched = first == 0 ? s->untouched : 0;
+    for (size_t i = 0; untouched && i < P->gates.size(); ++i)
+        if (!std::isfinite(P->gates[i].theta)) untouched = 0;    // zero times infinity would not stay zero
     s->untouched = 0;
     if ((r = qs_plan_upload(P, s))) return r;
     // Norm partials live in their own per-state buffer, so that other calls
@@ -921,6 +925,8 @@ extern "C" int qs_plan_apply_range(qs_state *s, qs_plan *P, size_t first, size_t
             const PlanPass &pp = P->passes[u];
             qs_tiled_desc &d = descs[u - first];
             d.threads_per_row = P->opts.threads_per_row;
+            for (int t = 0; t < 12; ++t) untouched &= ~(1ull << pp.T[t]);
+            d.zeros = untouched != 0;
             if (dst[u - first] >= 0) {
                 d.amp_out = buf[dst[u - first]];
                 d.amp_in = buf[dst[u - first] ^ 1];

@@ -254,6 +254,7 @@ struct TParams {
     const uint16_t *mat;         // nsub x [2][64][64] BF16 bits (hi, lo), the plan's column order
     int *err;
     int early;                   // the next kernel may be scheduled from this one's start
+    int zeros;                   // tiles of zeros are likely
     int nparts;                  // norm partials per pass (>= gridDim.x; the tail is written as zeros)
     const double *norm0;
     const double *prev_out;
@@ -392,6 +393,25 @@ __global__ void __launch_bounds__(TShape<TPR>::kCtaThreads, 1) k_tile_tmem(const
                 }
             }
             if (want_in) acc_in += (double)sum_squares(y);
+            if (P.zeros) {
+                // after |0...0>, with a qubit outside the tile still in |0>: a tile
+                // of zeros skips the blocks (30 qubits, the first three passes of a
+                // remapped plan)
+                bool any = false;
+#pragma unroll
+                for (int e = 0; e < kV; ++e) any = any || !(y[e] == 0.f);
+                if (!group_bar_or<S::kGroupThreads>(bar_id, any)) {
+                    if (amp != out) {
+                        const uint64_t obase = store_base(tile, tbase, P.W) | orow;
+#pragma unroll
+                        for (int j = 0; j < 32 / TPR; ++j)
+                            *reinterpret_cast<float2 *>(out + 2 * (obase | L.o_col[j])) = make_float2(0.f, 0.f);
+                    }
+                    if (tile + stride < P.tiles) copy_tile<TPR>(amp, tnext, L, stage, g_t, cs_t);
+                    tbase = tnext;
+                    continue;
+                }
+            }
             split_store<TPR>(tlane, y, c0);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -518,6 +538,7 @@ int qs_launch_tiled_tmem(qs_state *s, const qs_tiled_desc *d, int *err_dev)
     P.err = err_dev;
     // up to 25 qubits (24: 1.54 -> 1.51 ms for 31 passes; 21: 0.322 -> 0.294 ms
     // for 19); at 30 the next pass's early CTAs cost 1 %
+    P.zeros = d->zeros;
     P.early = P.tiles <= 16ull * QS_SM_COUNT * kGroups;
     P.nparts = qs_tiled_grid(s);
     P.norm0 = d->norm0;
