@@ -54,6 +54,24 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
     // nothing else lies between, the one before it
     int open[64], before[64];
     for (int q = 0; q < 64; ++q) open[q] = before[q] = -1;
+    // Gates on several qubits that touch a qubit close its last op, except
+    // where that op commutes with them: a diagonal op with controls and
+    // phases, an X-type op (a I + b X: RX) with the target of an X.  Only gates
+    // of the same type may then still join it (in layers of random rotations
+    // and CNOTs every ninth does).
+    uint64_t diag_only = 0, x_only = 0;
+    auto x_type = [](const double m[8]) { return m[0] == m[6] && m[1] == m[7] && m[2] == m[4] && m[3] == m[5]; };
+    auto close = [&](uint64_t qs, uint64_t z, uint64_t x) {      // z, x: the qubits of qs it acts on like Z, like X
+        for (; qs; qs &= qs - 1) {
+            const int q = low_bit(qs), o = open[q];
+            before[q] = -1;
+            if (o < 0) continue;
+            const uint64_t b = 1ull << q;
+            if ((z & b) && is_diag(ops[o].m) && !(x_only & b)) diag_only |= b;
+            else if ((x & b) && x_type(ops[o].m) && !(diag_only & b)) x_only |= b;
+            else open[q] = -1;
+        }
+    };
     int last_diag = -1;                    // the phase op that another phase may join ...
     uint64_t since = 0;                    // ... and the qubits mixed after it
     for (size_t i = 0; i < prims.size(); ++i) {
@@ -62,7 +80,9 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
             // Gates of one form multiply into one op.  Two of different forms
             // stay two ops: their product would be dense, 20 instructions per
             // pair against 6 + 5 for a rotation and a phase; three become one.
-            const int q = low_bit(p.off1), o = open[q];
+            const int q = low_bit(p.off1);
+            if (((diag_only >> q & 1) && !is_diag(p.m)) || ((x_only >> q & 1) && !x_type(p.m))) open[q] = -1;
+            const int o = open[q];
             if (o >= 0 && (form(ops[o].m) == form(p.m) || form(ops[o].m) == 3)) {
                 mul2(ops[o].m, p.m);
                 continue;
@@ -80,13 +100,15 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
             g.type = G_U;
             g.tgt = p.off1;
             memcpy(g.m, p.m, sizeof(g.m));
-            before[q] = o;
+            before[q] = (diag_only | x_only) >> q & 1 ? -1 : o;
             open[q] = (int)ops.size();
+            diag_only &= ~g.tgt;
+            x_only &= ~g.tgt;
             since |= g.tgt;
             ops.push_back(g);
             continue;
         }
-        for (uint64_t h = p.holes; h; h &= h - 1) open[low_bit(h)] = before[low_bit(h)] = -1;
+        close(p.holes, p.kind == QS_PRIM_PHASE ? p.holes : p.cmask, p.off0 == 0 && is_x(p.m) ? p.off1 : 0);
         if (p.kind == QS_PRIM_PHASE) {
             if (last_diag >= 0 && !(since & p.holes)) {
                 // join the last phase op when every term then has at most one
@@ -427,8 +449,11 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
             double best_gain = -1;
             for (uint32_t w : wants) {
                 if (w & ~allowed) continue;
+                // a tie goes to the lowest bits: left to the last stage with
+                // ops, they cost a stage of their own before the store
                 const double gain =
-                    (double)(scan(swaps ? todo : rest_of, regs | w, nullptr, nullptr, nullptr) - have) / popc(w);
+                    (double)(scan(swaps ? todo : rest_of, regs | w, nullptr, nullptr, nullptr) - have) / popc(w) +
+                    (w & low_tile ? 0.1 : 0);
                 if (gain > best_gain) { best_gain = gain; best = w; }
             }
             if (!best) break;
