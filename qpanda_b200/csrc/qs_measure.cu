@@ -120,7 +120,9 @@ struct MeasureResult {
 };
 
 // mode 0: res->p0 = sum; mode 1: measurement decision with uniform u.
-__global__ void k_finalize(const double *partials, int count, MeasureResult *res, int mode, double u)
+// host: the same result in the state's pinned host buffer (null: none).
+__global__ void k_finalize(const double *partials, int count, MeasureResult *res, MeasureResult *host, int mode,
+                           double u)
 {
     double acc = 0;
     for (int i = threadIdx.x; i < count; i += blockDim.x) acc += partials[i];
@@ -138,6 +140,7 @@ __global__ void k_finalize(const double *partials, int count, MeasureResult *res
             if (!(psel > 0.0)) res->status = 1;
             else res->scale = 1.0 / sqrt(psel);
         }
+        if (host) *host = *res;
     }
 }
 
@@ -526,6 +529,56 @@ __global__ void k_shots(const T *__restrict__ a, const double *__restrict__ tree
     }
 }
 
+// The whole sampler of a state of up to kSmallQubits qubits in one CTA: the
+// bins of the measured qubits, the outcome tree, then a thread per shot.
+// (256 shots of 9 qubits: four launches and their gaps, 61 us a call, most of
+// it spent around 15 us of kernels.)
+constexpr int kSmallQubits = 11;
+
+template <typename T>
+__global__ void __launch_bounds__(512)
+k_sample_small(const T *__restrict__ a, int n, int m, const __grid_constant__ ShotParams P,
+               const double *__restrict__ u, uint64_t shots, uint64_t *__restrict__ out)
+{
+    typedef typename vec2<T>::type V;
+    __shared__ double tree[2 << kSmallQubits];
+    const V *pa = reinterpret_cast<const V *>(a);
+    uint32_t free_bits = (1u << n) - 1;                        // the qubits that are not measured
+    for (int k = 0; k < m; ++k) free_bits &= ~(1u << P.qubits[k]);
+    for (uint32_t b = threadIdx.x; b < 1u << m; b += blockDim.x) {
+        uint32_t at = 0;
+        for (int k = 0; k < m; ++k) at |= (b >> k & 1u) << P.qubits[k];
+        double s = 0;
+        uint32_t w = 0;
+        do {                                                   // over the settings of the free bits, ascending
+            const V x = pa[at | w];
+            s += p2(x.x, x.y);
+            w = (w - free_bits) & free_bits;
+        } while (w);
+        tree[(1u << m) + b] = s;
+    }
+    for (int k = m - 1; k >= 0; --k) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < 1u << k; i += blockDim.x)
+            tree[(1u << k) + i] = tree[(2u << k) + i] + tree[(2u << k) + i + (1u << k)];
+    }
+    __syncthreads();
+    for (uint64_t s = threadIdx.x; s < shots; s += blockDim.x) {
+        uint32_t x = 0;
+        double S = 1.0;
+        for (int k = 0; k < m; ++k) {                          // k_shots' arithmetic
+            const double p0 = tree[(2u << k) + x] * S;
+            const float fi = (float)u[s * (uint64_t)m + k];
+            const int b = ((double)fi > p0) ? 1 : 0;
+            const double psel = b ? 1.0 - p0 : p0;
+            const double sc = 1.0 / sqrt(psel);
+            S *= sc * sc;
+            x |= (uint32_t)b << k;
+        }
+        out[s] = x;
+    }
+}
+
 // -------------------------------------------------------------- norm, inner
 template <typename Ta, typename Tb>
 __global__ void __launch_bounds__(kThreads)
@@ -611,17 +664,18 @@ k_diff(const Ta *__restrict__ a, const Tb *__restrict__ b, uint64_t N, double *p
     }
 }
 
-__global__ void k_finalize_diff(const double *partials, int count, double *res)
+__global__ void k_finalize_diff(const double *partials, int count, double *res, double *host)
 {
     if (threadIdx.x == 0) {
         double m = 0, s = 0;
         for (int i = 0; i < count; ++i) { m = fmax(m, partials[2 * i]); s += partials[2 * i + 1]; }
         res[0] = sqrt(m);
         res[1] = s;
+        if (host) { host[0] = sqrt(m); host[1] = s; }
     }
 }
 
-__global__ void k_finalize2(const double *partials, int count, double *res)
+__global__ void k_finalize2(const double *partials, int count, double *res, double *host)
 {
     double re = 0, im = 0;
     for (int i = threadIdx.x; i < count; i += blockDim.x) {
@@ -630,7 +684,10 @@ __global__ void k_finalize2(const double *partials, int count, double *res)
     }
     double r = block_sum(re);
     double s = block_sum(im);
-    if (threadIdx.x == 0) { res[0] = r; res[1] = s; }
+    if (threadIdx.x == 0) {
+        res[0] = r; res[1] = s;
+        if (host) { host[0] = r; host[1] = s; }
+    }
 }
 
 template <typename T>
@@ -661,9 +718,20 @@ int half_sum(qs_state *s, int q, int *nblocks)
     return QS_OK;
 }
 
+// Small results go straight into the state's pinned host buffer (4 KB), without
+// a copy behind the kernel; states with stream-ordered memory have none.
+constexpr size_t kPinned = 4096;
+
+template <typename R>
+R *pinned_out(const qs_state *s)
+{
+    return s->stream_alloc ? nullptr : static_cast<R *>(s->pinned);
+}
+
 int read_result(qs_state *s, size_t off, size_t bytes)
 {
-    QS_CUDA_TRY(cudaMemcpyAsync(s->pinned, static_cast<char *>(s->scratch) + off, bytes,
+    if (s->stream_alloc)
+        QS_CUDA_TRY(cudaMemcpyAsync(s->pinned, static_cast<char *>(s->scratch) + off, bytes,
                                 cudaMemcpyDeviceToHost, s->stream));
     QS_CUDA_TRY(cudaStreamSynchronize(s->stream));
     return QS_OK;
@@ -676,7 +744,7 @@ int prob_zero_t(qs_state *s, int q, double *p0)
     if ((r = half_sum<T>(s, q, &nb))) return r;
     double *part = reinterpret_cast<double *>(static_cast<char *>(s->scratch) + kPartOff);
     MeasureResult *res = reinterpret_cast<MeasureResult *>(static_cast<char *>(s->scratch) + kResOff);
-    k_finalize<<<1, kThreads, 0, s->stream>>>(part, nb, res, 0, 0.0);
+    k_finalize<<<1, kThreads, 0, s->stream>>>(part, nb, res, pinned_out<MeasureResult>(s), 0, 0.0);
     QS_LAUNCH_CHECK("k_finalize");
     if ((r = read_result(s, kResOff, sizeof(MeasureResult)))) return r;
     *p0 = static_cast<MeasureResult *>(s->pinned)->p0;
@@ -690,7 +758,7 @@ int measure_t(qs_state *s, int q, double u, int *outcome)
     if ((r = half_sum<T>(s, q, &nb))) return r;
     double *part = reinterpret_cast<double *>(static_cast<char *>(s->scratch) + kPartOff);
     MeasureResult *res = reinterpret_cast<MeasureResult *>(static_cast<char *>(s->scratch) + kResOff);
-    k_finalize<<<1, kThreads, 0, s->stream>>>(part, nb, res, 1, u);
+    k_finalize<<<1, kThreads, 0, s->stream>>>(part, nb, res, pinned_out<MeasureResult>(s), 1, u);
     QS_LAUNCH_CHECK("k_finalize");
     uint64_t pairs = s->N >> 1;
     k_collapse<T><<<grid_for(pairs, kThreads), kThreads, 0, s->stream>>>(static_cast<T *>(s->amp), pairs, q, res);
@@ -813,7 +881,13 @@ int probs_t(qs_state *s, const int *qubits, int m, double *out)
     if (r) return r;
     char *sc = static_cast<char *>(s->scratch);
     double *dev = reinterpret_cast<double *>(sc + kBufOff);
-    if ((r = marginal_launch<T>(s, P, dev, reinterpret_cast<double *>(sc + o_part)))) return r;
+    double *small = outb <= kPinned ? pinned_out<double>(s) : nullptr;
+    if ((r = marginal_launch<T>(s, P, small ? small : dev, reinterpret_cast<double *>(sc + o_part)))) return r;
+    if (small) {
+        QS_CUDA_TRY(cudaStreamSynchronize(s->stream));
+        memcpy(out, small, outb);
+        return QS_OK;
+    }
     QS_CUDA_TRY(cudaMemcpyAsync(out, dev, outb, cudaMemcpyDeviceToHost, s->stream));
     QS_CUDA_TRY(cudaStreamSynchronize(s->stream));
     return QS_OK;
@@ -834,6 +908,24 @@ int sample_t(qs_state *s, const int *qubits, int m, const double *u, size_t shot
     int r = qs_ensure_scratch(s, o_part + part_b);
     if (r) return r;
     char *sc = static_cast<char *>(s->scratch);
+    ShotParams SP;
+    for (int k = 0; k < m; ++k) SP.qubits[k] = (int8_t)qubits[k];
+    uint64_t *small = out_b <= kPinned ? pinned_out<uint64_t>(s) : nullptr;
+    uint64_t *res = small ? small : reinterpret_cast<uint64_t *>(sc + o_out);
+    auto finish = [&]() -> int {
+        if (!small) QS_CUDA_TRY(cudaMemcpyAsync(out, res, out_b, cudaMemcpyDeviceToHost, s->stream));
+        QS_CUDA_TRY(cudaStreamSynchronize(s->stream));
+        if (small) memcpy(out, small, out_b);
+        return QS_OK;
+    };
+    // (many shots are better spread over the device: k_shots)
+    if (s->n <= kSmallQubits && shots <= 4096) {
+        QS_CUDA_TRY(cudaMemcpyAsync(sc + o_u, u, u_b, cudaMemcpyHostToDevice, s->stream));
+        k_sample_small<T><<<1, 512, 0, s->stream>>>(static_cast<const T *>(s->amp), s->n, m, SP,
+                                                    reinterpret_cast<const double *>(sc + o_u), shots, res);
+        QS_LAUNCH_CHECK("k_sample_small");
+        return finish();
+    }
     double *tree = reinterpret_cast<double *>(sc + o_tree);
     // Level K0 = marginal over the first K0 measured qubits, stored at tree + 2^K0.
     if ((r = marginal_launch<T>(s, P, tree + (1ull << K0), reinterpret_cast<double *>(sc + o_part)))) return r;
@@ -845,8 +937,6 @@ int sample_t(qs_state *s, const int *qubits, int m, const double *u, size_t shot
     }
     k_fold_top<<<1, K0 < kFoldLow ? 256 : 1024, 0, s->stream>>>(tree, K0 < kFoldLow ? K0 : kFoldLow);
     QS_LAUNCH_CHECK("k_fold_top");
-    ShotParams SP;
-    for (int k = 0; k < m; ++k) SP.qubits[k] = (int8_t)qubits[k];
     for (int k = K0; k < m; ++k) {
         uint64_t mask = 0;
         for (int j = 0; j <= k; ++j) mask |= 1ull << qubits[j];
@@ -858,12 +948,9 @@ int sample_t(qs_state *s, const int *qubits, int m, const double *u, size_t shot
     unsigned grid = (unsigned)std::min<uint64_t>((warps_needed * 32 + thr - 1) / thr, (uint64_t)QS_SM_COUNT * 8);
     if (grid < 1) grid = 1;
     k_shots<T><<<grid, thr, 0, s->stream>>>(static_cast<const T *>(s->amp), tree, K0, m, SP,
-                                            reinterpret_cast<const double *>(sc + o_u), shots, s->n,
-                                            reinterpret_cast<uint64_t *>(sc + o_out));
+                                            reinterpret_cast<const double *>(sc + o_u), shots, s->n, res);
     QS_LAUNCH_CHECK("k_shots");
-    QS_CUDA_TRY(cudaMemcpyAsync(out, sc + o_out, out_b, cudaMemcpyDeviceToHost, s->stream));
-    QS_CUDA_TRY(cudaStreamSynchronize(s->stream));
-    return QS_OK;
+    return finish();
 }
 
 }  // namespace
@@ -933,7 +1020,7 @@ extern "C" int qs_norm2(qs_state *s, double *norm2)
     if (r) return r;
     double *part = reinterpret_cast<double *>(static_cast<char *>(s->scratch) + kPartOff);
     MeasureResult *res = reinterpret_cast<MeasureResult *>(static_cast<char *>(s->scratch) + kResOff);
-    k_finalize<<<1, kThreads, 0, s->stream>>>(part, nb, res, 0, 0.0);
+    k_finalize<<<1, kThreads, 0, s->stream>>>(part, nb, res, pinned_out<MeasureResult>(s), 0, 0.0);
     QS_LAUNCH_CHECK("k_finalize");
     if ((r = read_result(s, kResOff, sizeof(MeasureResult)))) return r;
     *norm2 = static_cast<MeasureResult *>(s->pinned)->p0;
@@ -960,7 +1047,7 @@ extern "C" int qs_inner(qs_state *a, qs_state *b, double *re, double *im)
         k_inner<double, double><<<grid, kThreads, 0, a->stream>>>((const double *)a->amp, (const double *)b->amp, a->N, part);
     QS_LAUNCH_CHECK("k_inner");
     double *res = reinterpret_cast<double *>(static_cast<char *>(a->scratch) + kResOff);
-    k_finalize2<<<1, kThreads, 0, a->stream>>>(part, (int)grid, res);
+    k_finalize2<<<1, kThreads, 0, a->stream>>>(part, (int)grid, res, pinned_out<double>(a));
     QS_LAUNCH_CHECK("k_finalize2");
     if ((r = read_result(a, kResOff, 16))) return r;
     *re = static_cast<double *>(a->pinned)[0];
@@ -987,7 +1074,7 @@ extern "C" int qs_diff(qs_state *a, qs_state *b, double *max_abs, double *sum_sq
         k_diff<double, double><<<grid, kThreads, 0, a->stream>>>((const double *)a->amp, (const double *)b->amp, a->N, part);
     QS_LAUNCH_CHECK("k_diff");
     double *res = reinterpret_cast<double *>(static_cast<char *>(a->scratch) + kResOff);
-    k_finalize_diff<<<1, 32, 0, a->stream>>>(part, (int)grid, res);
+    k_finalize_diff<<<1, 32, 0, a->stream>>>(part, (int)grid, res, pinned_out<double>(a));
     QS_LAUNCH_CHECK("k_finalize_diff");
     if ((r = read_result(a, kResOff, 16))) return r;
     if (max_abs) *max_abs = static_cast<double *>(a->pinned)[0];
