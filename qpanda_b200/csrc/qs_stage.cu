@@ -127,6 +127,66 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
     }
 }
 
+// Exchange amplitudes in place: see Permute (qs_stage.h).  Bound by HBM: one
+// read and one write of the state, in rows of at least 128 bytes on both
+// sides, however many pairs (the ten pairs that a 28-qubit QFT's last gate
+// pass leaves took three staged passes).
+template <typename T>
+__global__ void __launch_bounds__(256, 2) k_permute(T *__restrict__ a, const __grid_constant__ Permute P)
+{
+    constexpr int RB = Traits<T>::RB, NR = 1 << RB, LOW = Traits<T>::LOW;
+    typedef typename vec2<T>::type V;
+    extern __shared__ __align__(16) unsigned char stage_smem[];
+    V *tile = reinterpret_cast<V *>(stage_smem);
+    const uint32_t t = threadIdx.x;
+    qs_let_next_start();
+    const uint64_t base = tile_base(P, blockIdx.x), other = permute_partner(P, base);
+    if (base > other) return;                                  // the partner's CTA does both
+    uint32_t u = 0, w = 0, r = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        u += (t >> j & 1) * P.g_t[j];
+        w += (t >> j & 1) * P.w_t[j];
+        r += (t >> j & 1) * P.r_t[j];
+    }
+    V *here = reinterpret_cast<V *>(a) + base + (t & ((1u << LOW) - 1)) + ((uint64_t)u << LOW);
+    V *there = here + (other - base);
+    constexpr uint32_t kSlots = tile_slots<T>(RB + 8);
+    const bool two = other != base;
+    V x[NR], y[NR];
+    qs_wait_previous();
+#pragma unroll
+    for (int k = 0; k < NR; ++k) x[k] = here[(uint64_t)reg_sum<RB>(k, P.g_r) << LOW];
+    if (two) {
+#pragma unroll
+        for (int k = 0; k < NR; ++k) y[k] = there[(uint64_t)reg_sum<RB>(k, P.g_r) << LOW];
+    }
+#pragma unroll
+    for (int k = 0; k < NR; ++k) tile[w + reg_sum<RB>(k, P.w_r)] = x[k];
+    if (two) {
+#pragma unroll
+        for (int k = 0; k < NR; ++k) tile[kSlots + w + reg_sum<RB>(k, P.w_r)] = y[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NR; ++k) there[(uint64_t)reg_sum<RB>(k, P.g_r) << LOW] = tile[r + reg_sum<RB>(k, P.r_r)];
+    if (two) {
+#pragma unroll
+        for (int k = 0; k < NR; ++k) here[(uint64_t)reg_sum<RB>(k, P.g_r) << LOW] = tile[kSlots + r + reg_sum<RB>(k, P.r_r)];
+    }
+}
+
+template <typename T>
+int launch_permute(qs_state *s, const Permute &P)
+{
+    constexpr size_t smem = 2 * 2 * sizeof(T) * tile_slots<T>(Traits<T>::RB + 8);
+    QS_CUDA_TRY(cudaFuncSetAttribute(k_permute<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    QS_CUDA_TRY(qs_launch_overlapped(k_permute<T>, (unsigned)(s->N >> P.K), 1u << (P.K - Traits<T>::RB), smem,
+                                     s->stream, static_cast<T *>(s->amp), P));
+    QS_LAUNCH_CHECK("k_permute");
+    return QS_OK;
+}
+
 template <typename T, typename R>
 int launch(qs_state *s, const R &P)
 {
@@ -197,7 +257,13 @@ int apply_t(qs_state *s, const std::vector<qs_prim> &prims)
     bool finite = true;                          // zero times infinity would not stay zero
     for (const qs_prim &p : prims)
         for (int k = 0; s->untouched && k < 8; ++k) finite = finite && std::isfinite(p.m[k]);
-    while (P.next(&qmask, &pass)) {
+    Permute perm;
+    while (true) {
+        if (plan_permute<T>(P, &perm)) {
+            s->untouched = 0;
+            return launch_permute<T>(s, perm);
+        }
+        if (!P.next(&qmask, &pass)) break;
         // a pass that would move more than its gates one by one stays with them
         double traffic = 0;
         for (int i : pass) traffic += op_traffic(P, P.ops[(size_t)i]);

@@ -462,6 +462,38 @@ private:
     int scan(const std::vector<Masks> &list, uint64_t q, std::vector<uint64_t> *wants, std::vector<Masks> *kept) const;
 };
 
+// A list that ends in SWAPs of disjoint qubits (a QFT's reversal) ends in one
+// exchange of amplitudes in place, whatever the number of pairs (k_permute,
+// qs_stage.cu), where staged passes rename at most the qubits of a tile each.
+// A tile holds the lowest qubits, their partners and more pairs (or unpaired
+// qubits); with the tile's amplitudes at one setting of the other qubits go
+// those at the setting that the other pairs exchange it with.
+struct Permute {
+    int32_t K, nseg, npairs, pad;
+    uint64_t seg_mask[kMaxSeg];            // the tile index's bits (see Run)
+    uint64_t pair_a[16], pair_b[16];       // qubits outside the tile that trade places (2^q)
+    uint32_t g_t[kMaxThreadBits], g_r[4];  // state offsets of thread bits from LOW up and of register bits (see Run)
+    uint32_t w_t[kMaxThreadBits];          // slot weights of thread bits: written ...
+    uint32_t r_t[kMaxThreadBits];          // ... and read, at the partner's tile bit
+    uint32_t w_r[4], r_r[4];               // the same of register bits
+    uint8_t seg_shift[kMaxSeg + 3];
+};
+
+// The setting of the qubits outside the tile that base trades with.
+QS_HD uint64_t permute_partner(const Permute &P, uint64_t base)
+{
+    for (int j = 0; j < P.npairs; ++j) {
+        const bool a = (base & P.pair_a[j]) != 0, b = (base & P.pair_b[j]) != 0;
+        if (a != b) base ^= P.pair_a[j] | P.pair_b[j];
+    }
+    return base;
+}
+
+// True, and P, when the ops still left are SWAPs of disjoint pairs that staged
+// passes would take more than one pass for.
+template <typename T>
+bool plan_permute(const Planner &plan, Permute *P);
+
 // The stages of a pass (a RunSmall or RunLarge): fills R from pass_ops on the
 // tile of qmask; ops that do not fit R come back in *rest, in order.
 template <typename R, typename T>

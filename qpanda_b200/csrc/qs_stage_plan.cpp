@@ -274,6 +274,85 @@ void Planner::give_back(const std::vector<int> &rest)
     left.swap(all);
 }
 
+namespace {
+
+// The bits of a tile index in the qubits outside the tile, run by run; returns
+// the number of runs.
+int tile_segments(uint64_t qmask, int n, uint64_t *mask, uint8_t *shift)
+{
+    int nseg = 0;
+    for (int q = 0, from = 0; q < n;) {
+        if (qmask >> q & 1) { ++q; continue; }
+        int len = 0;
+        while (q + len < n && !(qmask >> (q + len) & 1)) ++len;
+        mask[nseg] = ((1ull << len) - 1) << from;
+        shift[nseg] = (uint8_t)(q - from);
+        ++nseg;
+        from += len;
+        q += len;
+    }
+    return nseg;
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------ the closing exchange
+template <typename T>
+bool plan_permute(const Planner &plan, Permute *P)
+{
+    constexpr int RB = Traits<T>::RB, LOW = Traits<T>::LOW;
+    constexpr int K = RB + 8;                          // 256 threads (128 when no bit is left without its partner)
+    const int n = plan.n;
+    if (n < K || plan.left.size() < 2 || plan.left.size() > 16 + K / 2) return false;
+    int partner[64];
+    for (int q = 0; q < n; ++q) partner[q] = q;
+    uint64_t all = 0;
+    for (int i : plan.left) {
+        const GOp &g = plan.ops[(size_t)i];
+        if (g.type != G_SWAP || (all & g.tgt)) return false;
+        all |= g.tgt;
+        const int a = low_bit(g.tgt), b = 63 - __builtin_clzll(g.tgt);
+        partner[a] = b;
+        partner[b] = a;
+    }
+    const uint64_t low = (1ull << LOW) - 1;
+    if (popc(all | low) <= plan.K) return false;       // one staged pass
+    // the tile: the lowest qubits and their partners, then pairs and unpaired
+    // qubits from the lowest up (rows of the state stay together)
+    uint64_t q = low;
+    for (int b = 0; b < LOW; ++b) q |= 1ull << partner[b];
+    for (int b = 0; b < n && popc(q) < K; ++b) {
+        const uint64_t add = (1ull << b | 1ull << partner[b]) & ~q;
+        if (popc(q | add) <= K) q |= add;
+    }
+    if (popc(q) < K - 1) return false;
+    memset(P, 0, sizeof(*P));
+    P->K = popc(q);
+    P->nseg = tile_segments(q, n, P->seg_mask, P->seg_shift);
+    for (int a = 0; a < n; ++a)
+        if (partner[a] > a && !(q >> a & 1)) {
+            if (P->npairs == 16) return false;
+            P->pair_a[P->npairs] = 1ull << a;
+            P->pair_b[P->npairs++] = 1ull << partner[a];
+        }
+    int pos[64], k = 0;
+    for (int b = 0; b < n; ++b)
+        if (q >> b & 1) pos[b] = k++;
+    for (int b = 0; b < n; ++b) {
+        if (!(q >> b & 1)) continue;
+        const int at = pos[b];
+        const bool thread = at < P->K - RB;
+        const int j = thread ? at : at - (P->K - RB);
+        (thread ? P->w_t : P->w_r)[j] = slot_weight<T>(at);
+        (thread ? P->r_t : P->r_r)[j] = slot_weight<T>(pos[partner[b]]);
+        if (at >= LOW) (thread ? P->g_t : P->g_r)[j] = 1u << (b - LOW);
+    }
+    return true;
+}
+
+template bool plan_permute<float>(const Planner &, Permute *);
+template bool plan_permute<double>(const Planner &, Permute *);
+
 // ------------------------------------------------------------------ stages of a pass
 namespace {
 
@@ -350,18 +429,7 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
             }
         }
     }
-    // the tile index's bits go to the qubits outside the tile, run by run
-    S.nseg = 0;
-    for (int q = 0, from = 0; q < n;) {
-        if (qmask >> q & 1) { ++q; continue; }
-        int len = 0;
-        while (q + len < n && !(qmask >> (q + len) & 1)) ++len;
-        S.seg_mask[S.nseg] = ((1ull << len) - 1) << from;
-        S.seg_shift[S.nseg] = (uint8_t)(q - from);
-        ++S.nseg;
-        from += len;
-        q += len;
-    }
+    S.nseg = tile_segments(qmask, n, S.seg_mask, S.seg_shift);
     auto tile_bits = [&](uint64_t qs, const int *ps) {
         uint32_t o = 0;
         for (qs &= qmask; qs; qs &= qs - 1) o |= 1u << ps[low_bit(qs)];

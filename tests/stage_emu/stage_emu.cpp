@@ -146,6 +146,51 @@ int run_pass(std::vector<V2<T>> &a, int n, const R &P, Stats &st)
 }
 
 template <typename T>
+int run_permute(std::vector<V2<T>> &a, const Permute &P, Stats &st)
+{
+    constexpr int RB = Traits<T>::RB, NR = 1 << RB, LOW = Traits<T>::LOW;
+    constexpr uint32_t slots_n = tile_slots<T>(RB + 8);
+    const uint32_t threads = 1u << (P.K - RB);
+    if (P.K != RB + 8 && P.K != RB + 7) return fail("permute tile %lld", P.K);
+    std::vector<uint8_t> seen(a.size(), 0), stored(a.size(), 0);
+    std::vector<V2<T>> out(a), tile(2 * slots_n);
+    for (uint64_t tl = 0; tl < a.size() >> P.K; ++tl) {
+        const uint64_t base = tile_base(P, tl), other = permute_partner(P, base);
+        if (permute_partner(P, other) != base) return fail("tile %lld has no partner", (long long)tl);
+        if (base > other) continue;
+        const int two = other != base;
+        std::vector<uint8_t> wr(2 * slots_n, 0), rd(2 * slots_n, 0);
+        for (int store = 0; store < 2; ++store)
+            for (int side = 0; side <= two; ++side)
+                for (int k = 0; k < NR; ++k) {
+                    std::vector<uint32_t> slots(threads);
+                    for (uint32_t t = 0; t < threads; ++t) {
+                        uint32_t u = 0, w = 0;
+                        for (int j = 0; j < 8; ++j) {
+                            u += (t >> j & 1) * P.g_t[j];
+                            w += (t >> j & 1) * (store ? P.r_t[j] : P.w_t[j]);
+                        }
+                        const uint32_t sl = side * slots_n + w + reg_sum<RB>(k, store ? P.r_r : P.w_r);
+                        const uint64_t at = ((store ? !side : side) && two ? other : base) + (t & ((1u << LOW) - 1)) +
+                                            ((uint64_t)(u + reg_sum<RB>(k, P.g_r)) << LOW);
+                        if (at >= a.size() || sl >= 2 * slots_n || (store ? stored : seen)[at]++ || (store ? rd : wr)[sl]++)
+                            return fail("amplitude %lld or slot %lld used twice", (long long)at, sl);
+                        if (store && (!seen[at] || !wr[sl])) return fail("amplitude %lld stored before its load", (long long)at);
+                        if (store) out[at] = tile[sl];
+                        else tile[sl] = a[at];
+                        slots[t] = sl;
+                    }
+                    st.conflicts += conflicts(slots, 1 << Traits<T>::LB);
+                }
+    }
+    for (size_t i = 0; i < a.size(); ++i)
+        if (seen[i] != 1 || stored[i] != 1) return fail("amplitude %lld missed", (long long)i);
+    a.swap(out);
+    ++st.passes;
+    return 0;
+}
+
+template <typename T>
 int run(double *amp, int n, const std::vector<qs_prim> &prims, int dtype, bool execute, Stats &st)
 {
     std::vector<V2<T>> a(execute ? (size_t)1 << n : 0);
@@ -156,7 +201,14 @@ int run(double *amp, int n, const std::vector<qs_prim> &prims, int dtype, bool e
     auto S = new RunSmall<T>();
     auto L = new RunLarge<T>();
     int r = 0;
-    while (!r && P.next(&qmask, &pass)) {
+    Permute perm;
+    while (!r) {
+        if (plan_permute<T>(P, &perm)) {
+            if (execute) r = run_permute<T>(a, perm, st);
+            else ++st.passes;
+            break;
+        }
+        if (!P.next(&qmask, &pass)) break;
         bool done = false;
         if ((int)pass.size() < RunSmall<T>::NOP - 1) {
             plan_pass<RunSmall<T>, T>(P, qmask, pass, S, &rest);

@@ -9,7 +9,7 @@ import pytest
 from oracle.pyoracle import OracleState
 from qpanda_b200 import StateVector, circuits
 from qpanda_b200.capi import check, lib
-from tests.test_stage_emulation import LISTS
+from tests.test_stage_emulation import LISTS, swaps
 
 pytestmark = pytest.mark.gpu
 
@@ -84,3 +84,18 @@ def test_lists_from_zero_state(need_gpu, n, dtype):
         o.set_state(init)
         o.apply(gates)
         assert np.abs(got - o.state()).max() < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("n", [13, 16, 19])
+@pytest.mark.parametrize("kind", ["all", "upper", "random"])
+def test_closing_exchange(need_gpu, kind, n, dtype):
+    init, gates = random_state(n, n), swaps(n, kind)
+    with StateVector(n, dtype) as sv:
+        sv.set_state(init.astype(np.complex64) if dtype == "c64" else init)
+        sv.apply(gates)
+        got = sv.get_state()
+    o = OracleState(n)
+    o.set_state(init)
+    o.apply(gates)
+    assert np.abs(got - o.state()).max() < TOL[dtype]
