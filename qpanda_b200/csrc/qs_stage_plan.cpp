@@ -171,6 +171,18 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
         g.tgt = 0;
         g.type = G_DIAG;
     }
+    // a ladder runs where its hub is mixed next (as one op with an H): it counts
+    // as a gate on the hub, or it would run as soon as its qubits are ready, on
+    // tiles and threads that half of the time have the hub clear
+    uint64_t mixed = 0;                    // qubits that a 1-qubit op mixes next
+    for (size_t i = ops.size(); i-- > 0;) {
+        GOp &g = ops[i];
+        if (g.type == G_NONE) continue;
+        const bool ladder = g.type == G_DIAG && g.count > 1 && popc(g.ctrl) == 1;
+        if (ladder && (g.ctrl & mixed)) g.tgt = g.ctrl;
+        if (g.type == G_U) mixed |= g.tgt;
+        else if (!ladder) mixed &= ~(g.tgt | g.diag);
+    }
     left.reserve(ops.size());
     for (size_t i = 0; i < ops.size(); ++i)
         if (ops[i].type != G_NONE) left.push_back((int)i);
@@ -598,9 +610,18 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         memset(&op, 0, sizeof(op));
         if (g.type == G_U) {
             double p;
-            op.kind = (uint8_t)(classify<T>(g.m, op.m, &p) + reg_bit(g.tgt));
+            const int j = reg_bit(g.tgt);
+            const uint8_t kind = classify<T>(g.m, op.m, &p);
             scale *= p;
             growth /= std::fabs(p);
+            // an H right behind the ladder whose hub it mixes: one op
+            Op<T> *last = nops > S.st[S.nstages - 1].first ? &S.op[nops - 1] : nullptr;
+            if (kind == K_RAM && op.m[0] == 1 && op.m[1] == 1 && last && last->kind == K_LAD + j && !last->cond) {
+                last->kind = (uint8_t)(K_LADH + j);
+                --nops;                            // counted again below
+            } else {
+                op.kind = (uint8_t)(kind + j);
+            }
         } else if (g.type == G_CU) {
             condition(g.ctrl, &op);
             for (int k = 0; k < 8; ++k) op.m[k] = (T)g.m[k];
@@ -631,17 +652,16 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
             for (int side = 0; side < 2; ++side)
                 for (int k = 0; k < g.count; ++k) {
                     const Term &t = P.terms[(size_t)(g.first + k)];
-                    // a term on the hub alone: any of the hub's qubits carries it
-                    const int q = t.q >= 0 ? t.q : low_bit(g.ctrl);
-                    const bool out_q = outside >> q & 1;
-                    if (!out_q && reg_of[pos[q]] >= 0) {
+                    const bool alone = t.q < 0;              // on the hub alone
+                    const bool out_q = alone || (outside >> t.q & 1);
+                    if (!out_q && reg_of[pos[t.q]] >= 0) {
                         if (side) continue;
-                        T *w = &op.m[2 * reg_of[pos[q]]];
+                        T *w = &op.m[2 * reg_of[pos[t.q]]];
                         const cd z = cd(t.re, t.im) * cd((double)w[0], (double)w[1]);
                         w[0] = (T)z.real();
                         w[1] = (T)z.imag();
                     } else if (out_q == (side == 1)) {
-                        S.ent[nent++] = {t.re, t.im, out_q ? q : thread_of[pos[q]], 0};
+                        S.ent[nent++] = {t.re, t.im, alone ? -1 : out_q ? t.q : thread_of[pos[t.q]], 0};
                         ++(out_q ? L.nout : L.nthr);
                     }
                 }

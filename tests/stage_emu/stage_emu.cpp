@@ -107,7 +107,7 @@ int run_pass(std::vector<V2<T>> &a, int n, const R &P, Stats &st)
             for (int o = sg.first; o < sg.first + sg.count; ++o) {
                 if (o >= R::NOP) return fail("op %lld past the block", o);
                 const Op<T> &op = P.op[o];
-                if (op.kind >= K_LADR && op.kind <= K_LAD0 && op.ladder >= P.nladders) return fail("ladder %lld", op.ladder);
+                if (((op.kind >= K_LADR && op.kind <= K_LAD0) || op.kind >= K_LADH) && (int)op.ladder >= P.nladders) return fail("ladder %lld", op.ladder);
                 if (!op.cond && (op.need || op.cthr)) return fail("op %lld hides its condition", o);
                 if ((base & op.need) != op.need) continue;
                 for (uint32_t t = 0; t < threads; ++t) {
