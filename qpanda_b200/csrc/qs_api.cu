@@ -77,6 +77,17 @@ int qs_ensure_scratch(qs_state *s, size_t bytes)
     if (!s->stream_alloc) QS_CUDA_TRY(cudaStreamSynchronize(s->stream));
     int r = qs_dev_alloc(s, nb, &p);
     if (r) return r;
+    // the result words (64 KB in) keep what they hold - the fused passes' error
+    // word may not have been read yet - and start at zero
+    char *results = static_cast<char *>(p) + 64 * 1024;
+    const cudaError_t e = s->scratch ? cudaMemcpyAsync(results, static_cast<char *>(s->scratch) + 64 * 1024, 256,
+                                                       cudaMemcpyDeviceToDevice, s->stream)
+                                     : cudaMemsetAsync(results, 0, 256, s->stream);
+    if (e != cudaSuccess) {
+        qs_dev_free(s, p);
+        return qs_cuda_fail(e, "scratch");
+    }
+    if (s->scratch && !s->stream_alloc) QS_CUDA_TRY(cudaStreamSynchronize(s->stream));
     qs_dev_free(s, s->scratch);
     s->scratch = p;
     s->scratch_bytes = nb;

@@ -855,6 +855,10 @@ extern "C" int qs_plan_apply_range(qs_state *s, qs_plan *P, size_t first, size_t
     if (r) return r;
     if (!P) return qs_fail(QS_ERR_ARG, "qs_plan_apply: null plan");
     if (P->n != s->n) return qs_fail(QS_ERR_ARG, "qs_plan_apply: plan for %d qubits, state has %d", P->n, s->n);
+    // watchdog flag (result area of scratch), cleared before the first block
+    const size_t kFlagOff = 64 * 1024 + 192;
+    int *flag = reinterpret_cast<int *>(static_cast<char *>(s->scratch) + kFlagOff);
+    if (first == 0) QS_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), s->stream));
     if (s->dtype != QS_C64 || s->n < 12) {
         // No tensor-core form for complex128 or below 12 qubits: the gates of
         // the requested blocks (all gates when the plan has no blocks) through
@@ -896,10 +900,6 @@ extern "C" int qs_plan_apply_range(qs_state *s, qs_plan *P, size_t first, size_t
         s->fused_norm = static_cast<double *>(p);
     }
     double *norm = s->fused_norm;
-    // watchdog flag (result area of scratch), cleared before the first block
-    const size_t kFlagOff = 64 * 1024 + 192;
-    int *flag = reinterpret_cast<int *>(static_cast<char *>(s->scratch) + kFlagOff);
-    if (first == 0) QS_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), s->stream));
     const size_t per = 2 * 64 * 64 * sizeof(uint16_t);
     if (P->opts.kernel == QS_PLAN_TILED) {
         const int GT = qs_tiled_grid(s);
