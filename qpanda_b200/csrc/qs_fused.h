@@ -61,7 +61,10 @@ struct qs_tiled_desc {
     int threads_per_row;         // 1: 128 threads per lane, a row each; 2: 256, half a row each
 };
 
+// Norm partials per tiled pass: the largest grid of the tiled kernels.
 int qs_tiled_grid(const qs_state *s);
+// CTAs of one pass on k_tile_tmem (qs_tile_tmem.cu).
+int qs_tmem_grid(const qs_state *s);
 // Row-bit orders for a pass's blocks that keep warp-wide accesses coalesced
 // and the shared-memory stores free of bank conflicts as far as possible
 // (qs_tile_layout.cu).  rows[b][i] = global qubit of row bit i.  wtile: the

@@ -36,6 +36,8 @@
 // 0's B operand when the CTA loads it, and the input norm is accumulated only
 // on the plan's first pass (the only one whose input norm is used).
 // Bounded waits as in qs_fused.cu.
+#include <algorithm>
+
 #include "qs_fused.h"
 #include "qs_tile_core.cuh"
 
@@ -324,8 +326,8 @@ int launch(qs_state *s, const float *in, float *out, TileParams &P)
 
 int qs_tiled_grid(const qs_state *s)
 {
-    const uint64_t a = grid_for<2>(s), b = grid_for<3>(s);
-    return (int)(a > b ? a : b);                      // the larger of the two grids
+    // the largest grid of the kernels that may run a pass
+    return (int)std::max({(uint64_t)grid_for<2>(s), (uint64_t)grid_for<3>(s), (uint64_t)qs_tmem_grid(s)});
 }
 
 int qs_launch_tiled(qs_state *s, const qs_tiled_desc *d, int *err_dev)
