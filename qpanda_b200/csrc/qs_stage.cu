@@ -53,7 +53,7 @@ k_stage(T *__restrict__ a, const __grid_constant__ R P)
     }
     // the ladders' factors, while the loads are in flight
     V *lane_f = tile + tile_slots<T>(P.K), *warp_f = lane_f + 32 * P.nladders;
-    const uint32_t lw = P.K - RB - 5;                          // log2 of the CTA's warps
+    const uint32_t lw = warp_bits<T>(P.K);
     if (P.nladders) {
         for (uint32_t i = t; i < 32u * P.nladders; i += blockDim.x) {
             double fr, fi;
@@ -190,14 +190,14 @@ int launch_permute(qs_state *s, const Permute &P)
 template <typename T, typename R>
 int launch(qs_state *s, const R &P)
 {
-    const size_t amps = tile_slots<T>(P.K) + (size_t)P.nladders * (32 + (1u << (P.K - Traits<T>::RB - 5)));
+    const size_t amps = tile_slots<T>(P.K) + (size_t)P.nladders * (32 + (1u << warp_bits<T>(P.K)));
     const size_t smem = 2 * sizeof(T) * amps;
     if (smem > 48 * 1024) {
         // once per device and kernel: the largest a pass can need
         static std::atomic<uint64_t> done{0};
         const uint64_t bit = 1ull << (s->device & 63);
         if (!(done.load() & bit)) {
-            const int most = (int)(2 * sizeof(T) * (tile_slots<T>(kMaxTile) + R::NLAD * (32 + (1u << (kMaxTile - Traits<T>::RB - 5)))));
+            const int most = (int)(2 * sizeof(T) * (tile_slots<T>(kMaxTile) + R::NLAD * (32 + (1u << warp_bits<T>(kMaxTile)))));
             QS_CUDA_TRY(cudaFuncSetAttribute(k_stage<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
             done.fetch_or(bit);
         }

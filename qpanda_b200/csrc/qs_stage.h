@@ -55,7 +55,9 @@
 namespace qs_stg {
 
 constexpr int kMaxTile = 12;         // tile qubits
-constexpr int kMinTile = 9;          // narrower states stay on k_lowstage
+// Narrower states stay on k_lowstage (48 gates of 8 qubits: 54 us there, 42
+// here; of 6 and 7 qubits 47 and 49 on both).
+constexpr int kMinTile = 8;
 constexpr int kMaxThreadBits = 9;
 constexpr int kMaxSeg = kMaxTile + 1;
 
@@ -163,6 +165,13 @@ constexpr uint32_t tile_slots(int K)
     uint32_t n = 1;
     for (int b = 0; b < K; ++b) n += slot_weight<T>(b);
     return n;
+}
+
+// log2 of a CTA's warps (narrow tiles: part of one)
+template <typename T>
+QS_HD int warp_bits(int K)
+{
+    return K - Traits<T>::RB > 5 ? K - Traits<T>::RB - 5 : 0;
 }
 
 template <typename R>

@@ -23,7 +23,7 @@ def random_state(n, seed):
 
 
 @pytest.mark.parametrize("dtype", ["c64", "c128"])
-@pytest.mark.parametrize("n", [8, 9, 11, 12, 13, 17])
+@pytest.mark.parametrize("n", [7, 8, 9, 11, 12, 13, 17])
 @pytest.mark.parametrize("kind", list(LISTS))
 def test_lists_match_oracle(need_gpu, kind, n, dtype):
     init, gates = random_state(n, n), LISTS[kind](n)

@@ -76,7 +76,7 @@ LISTS = {
 
 
 @pytest.mark.parametrize("dtype", [C64, C128])
-@pytest.mark.parametrize("n", [9, 10, 12, 13, 15])
+@pytest.mark.parametrize("n", [8, 9, 10, 12, 13, 15])
 @pytest.mark.parametrize("kind", list(LISTS))
 def test_passes_match_oracle(emu, kind, n, dtype):
     rng = np.random.default_rng(7 * n + dtype)
