@@ -340,11 +340,18 @@ __global__ void __launch_bounds__(kThreads, BShape<SUB>::kCtasPerSm) k_batch(Bat
 // The same sweep with the tile in tensor memory: k_tile_tmem's pass body
 // (qs_tile_tmem.cu: staging copies in tile order, the row gather, the tile as
 // the MMAs' A operand in TMEM, the exchange between blocks through the staging
-// buffer, the stores of the last block) run by one 128-thread CTA per circuit,
-// three CTAs per SM, passes of up to two blocks; what k_batch adds stays as it
-// is: the queue, |0...0> on the first pass without reading memory, the
-// previous pass's norm folded into the first block's matrix, and the
-// <Z_i Z_{i+1}> of the last pass's output.
+// buffer, the stores of the last block) run by one CTA per circuit, passes of up
+// to two blocks; what k_batch adds stays as it is: the queue, |0...0> on the
+// first pass without reading memory, the previous pass's norm folded into the
+// first block's matrix, and the <Z_i Z_{i+1}> of the last pass's output.
+//
+// What bounds it is the chain of one tile (copy, gather, MMAs, exchange, MMAs,
+// store: 16 ns per tile and pass with three chains per SM, 10 ns at the HBM
+// rate for states past L2), so the tiles in flight per SM count.  A chain
+// needs 32 KB of staging and its matrices' 32 KB: three CTAs of 128 threads
+// per SM, or two CTAs of two such lane groups that share the matrices and walk
+// a circuit's tiles in turn (tm_groups has the rule; 256 circuits of 10..22
+// qubits: 7.6 -> 6.9 ms).
 //
 // A circuit that would keep one CTA busy past the others' end is shared: its
 // passes are cut into parts of a few tiles, each a task of the queue.  A part
@@ -355,18 +362,24 @@ __global__ void __launch_bounds__(kThreads, BShape<SUB>::kCtasPerSm) k_batch(Bat
 // (256 circuits of 10..22 qubits, 4..12 layers: one CTA per circuit took what
 // the deepest 22-qubit circuit takes, 96.6 ms; shared, 8.9 ms with the same
 // bits.  16 circuits of 20..22 qubits: 96.7 -> 3.9 ms.)
-constexpr int kTmThreads = 128;
-constexpr int kTmCtasPerSm = 3;
-constexpr uint32_t kTmOffB = 0;                                      // 2 blocks x (hi, lo) x 8 KB
-constexpr uint32_t kTmOffStage = 2 * 2 * kB;                         // 32 KB of staging
-constexpr uint32_t kTmOffLayout = kTmOffStage + kStage;
-constexpr uint32_t kTmLayoutBytes = (sizeof(qs_tmem::TLayout) + 15) & ~15u;
-constexpr uint32_t kTmOffMisc = kTmOffLayout + kTmLayoutBytes;       // mbarrier 8, tmem 4, circuit 4
-constexpr uint32_t kTmSmemBytes = kTmOffMisc + 16;
-constexpr uint32_t kTmCols = 128;
-static_assert(kTmCtasPerSm * (kTmSmemBytes + 1024) <= 228 * 1024, "resident CTAs per SM");
-static_assert(kTmCtasPerSm * kTmCols <= 512, "TMEM columns per SM");
-static_assert((4 + 4 * kMaxZZ) * 8 <= kStage, "reductions fit the staging buffer");
+//
+// GROUPS lane groups per CTA, each with its own staging buffer, mbarrier, named
+// barrier and 128 TMEM columns.
+template <int GROUPS>
+struct TmShape {
+    static constexpr int kThreads = 128 * GROUPS;
+    static constexpr int kCtasPerSm = GROUPS == 1 ? 3 : 2;
+    static constexpr uint32_t kOffB = 0;                                 // 2 blocks x (hi, lo) x 8 KB
+    static constexpr uint32_t kOffStage = 2 * 2 * kB;                    // 32 KB of staging per group
+    static constexpr uint32_t kOffLayout = kOffStage + GROUPS * kStage;
+    static constexpr uint32_t kLayoutBytes = (sizeof(qs_tmem::TLayout) + 15) & ~15u;
+    static constexpr uint32_t kOffMisc = kOffLayout + kLayoutBytes;      // mbarriers 8 each, tmem 4, circuit 4
+    static constexpr uint32_t kSmemBytes = kOffMisc + 32;
+    static constexpr uint32_t kCols = 128 * GROUPS;
+    static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "resident CTAs per SM");
+    static_assert(kCtasPerSm * kCols <= 512, "TMEM columns per SM");
+    static_assert(4 * GROUPS * (1 + kMaxZZ) * 8 <= kStage, "reductions fit a staging buffer");
+};
 
 // a warp's sum of n values that other CTAs wrote, in a fixed order
 __device__ __forceinline__ double sum_parts(const double *v, int stride, int n)
@@ -389,6 +402,45 @@ __device__ __forceinline__ bool all_zero(const float (&y)[64])
     return zero;
 }
 
+// A row's part of <Z_i Z_{i+1}>.  The sign of a pair is the parity of its two
+// bits, and at most two of them are register bits: one Walsh-Hadamard
+// transform of the row's 32 probabilities holds every pair's sum (160 adds
+// instead of 32 per pair), its sign follows from the row's own bits.  (Signed
+// sums per pair took a fifth of narrow sweeps: 1024 circuits of 4..12 qubits
+// 0.238 -> 0.180 ms, 256 of 10..22 7.97 -> 7.58.)
+__device__ __forceinline__ void add_zz(double (&zz)[kMaxZZ], float (&y)[64], uint64_t obase, const qs_tmem::TLayout &L,
+                                       int nzz)
+{
+    float s[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) s[j] = fmaf(y[2 * j], y[2 * j], y[2 * j + 1] * y[2 * j + 1]);
+#pragma unroll
+    for (int b = 0; b < 5; ++b)
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if (!((j >> b) & 1)) {
+                const float u = s[j], v = s[j | (1 << b)];
+                s[j] = u + v;
+                s[j | (1 << b)] = u - v;
+            }
+    uint32_t in[5];                                  // bit i: register bit b belongs to pair i
+#pragma unroll
+    for (int b = 0; b < 5; ++b) in[b] = (uint32_t)(L.o_col[1 << b] | (L.o_col[1 << b] >> 1));
+    const uint32_t all = (1u << nzz) - 1u, sign = (uint32_t)(obase ^ (obase >> 1));
+#pragma unroll
+    for (int m = 0; m < 32; ++m) {
+        if (__popc(m) > 2) continue;
+        uint32_t set = all;                          // the pairs with exactly these register bits
+#pragma unroll
+        for (int b = 0; b < 5; ++b) set &= (m >> b) & 1 ? in[b] : ~in[b];
+        while (set) {
+            const int i = __ffs(set) - 1;
+            set &= set - 1;
+            zz[i] += (double)__uint_as_float(__float_as_uint(s[m]) ^ (((sign >> i) & 1u) << 31));
+        }
+    }
+}
+
 // Wait until `need` parts of a circuit are done; false when that took longer
 // than any task can (2 s) or another CTA has failed.
 __device__ bool wait_parts(const int32_t *done, int32_t need, const int *err)
@@ -405,36 +457,42 @@ __device__ bool wait_parts(const int32_t *done, int32_t need, const int *err)
     }
 }
 
-__global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchParams P)
+template <int GROUPS>
+__global__ void __launch_bounds__(TmShape<GROUPS>::kThreads, TmShape<GROUPS>::kCtasPerSm) k_batch_tmem(BatchParams P)
 {
     namespace D = qs_tmem_dev;
+    using S = TmShape<GROUPS>;
+    constexpr int kTmThreads = S::kThreads, kWarps = kTmThreads / 32;
+    constexpr uint32_t kTmOffB = S::kOffB, kTmCols = S::kCols;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int grp = tid >> 7, ltid = tid & 127, wq = warp & 3, bar = 1 + grp;
     if (smem_u32(smem) & 1023u) {
         if (tid == 0) atomicExch(P.err, 2);
         return;
     }
-    qs_tmem::TLayout &L = *reinterpret_cast<qs_tmem::TLayout *>(smem + kTmOffLayout);
-    const uint32_t stage = smem_u32(smem + kTmOffStage);
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kTmOffMisc);
-    uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + kTmOffMisc + 8);
-    int32_t *s_circ = reinterpret_cast<int32_t *>(smem + kTmOffMisc + 12);
-    double *red = reinterpret_cast<double *>(smem + kTmOffStage);   // when no copy is in flight
+    qs_tmem::TLayout &L = *reinterpret_cast<qs_tmem::TLayout *>(smem + S::kOffLayout);
+    const uint32_t stage = smem_u32(smem + S::kOffStage + grp * kStage);
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + S::kOffMisc) + grp;
+    uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + S::kOffMisc + 16);
+    int32_t *s_circ = reinterpret_cast<int32_t *>(smem + S::kOffMisc + 20);
+    double *red = reinterpret_cast<double *>(smem + S::kOffStage);  // when no copy is in flight
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_u32(tmem_holder)), "r"(kTmCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    if (tid == 0) {
+    if (ltid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(mbar)), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tgrp = *tmem_holder;
-    const uint32_t tlane = tgrp + ((uint32_t)(warp * 32) << 16);
+    const uint32_t tmem = *tmem_holder;
+    const uint32_t tgrp = tmem + (uint32_t)(grp * 128);              // the group's 128 columns
+    const uint32_t tlane = tgrp + ((uint32_t)(wq * 32) << 16);
     const uint32_t mb = smem_u32(mbar);
     uint32_t phase = 0;
     bool failed = false;
@@ -482,7 +540,7 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
             // per-thread parts of the gather, exchange, copy and store addresses
             uint32_t xrow = 0, xw0 = 0, xr0 = 0;
             uint64_t orow = 0, g_t = 0;
-            uint32_t cs_t = (uint32_t)tid;
+            uint32_t cs_t = (uint32_t)ltid;
 #pragma unroll
             for (int i = 0; i < 5; ++i)
                 if ((lane >> i) & 1) {
@@ -493,7 +551,7 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                 }
 #pragma unroll
             for (int v = 0; v < 2; ++v)
-                if ((warp >> v) & 1) {
+                if ((wq >> v) & 1) {
                     xrow ^= L.s_warp[v];
                     orow |= L.o_warp[v];
                     xw0 ^= L.xw_warp[0][v];
@@ -501,23 +559,23 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                 }
 #pragma unroll
             for (int b = 0; b < 7; ++b)
-                if ((tid >> b) & 1) { g_t |= L.g_bit[b]; cs_t ^= L.cf_bit[b]; }
+                if ((ltid >> b) & 1) { g_t |= L.g_bit[b]; cs_t ^= L.cf_bit[b]; }
             const bool last_pass = p + 1 == C.npass;
             double acc_out = 0;
-            const uint64_t step = D::tbase_of(1, L);
-            uint64_t tbase = shared ? D::tbase_of(tile0, L) : 0;
-            if (p > 0) D::copy_tile<1>(C.amp, tbase, L, stage, g_t, cs_t);
-            for (uint64_t tile = tile0; tile < tiles; ++tile) {
+            const uint64_t step = D::tbase_of(GROUPS, L);
+            uint64_t tile = tile0 + grp, tbase = D::tbase_of(tile, L);
+            if (p > 0 && tile < tiles) D::copy_tile<1>(C.amp, tbase, L, stage, g_t, cs_t);
+            for (; tile < tiles; tile += GROUPS) {
                 const uint64_t tnext = tile_base_advance(tbase, step, L.tmask);
                 float y[64];
                 if (p == 0) {
                     // |0...0>: amplitude 0 is tile 0, the row with no row bits, column 0
 #pragma unroll
                     for (int e = 0; e < 64; ++e) y[e] = 0.f;
-                    if (tile == 0 && tid == 0) y[0] = 1.f;
+                    if (tile == 0 && ltid == 0) y[0] = 1.f;
                 } else {
                     asm volatile("cp.async.wait_group 0;" ::: "memory");
-                    __syncthreads();
+                    D::group_bar<128>(bar);
                     if (L.pair_in) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
@@ -531,7 +589,7 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                                          : "=f"(y[2 * j]), "=f"(y[2 * j + 1]) : "r"(stage + ((xrow ^ L.s_col[j]) << 3)));
                     }
                 }
-                if (zeros && !__syncthreads_or(!all_zero(y))) {
+                if (zeros && !D::group_bar_or<128>(bar, !all_zero(y))) {
                     // a tile of zeros: written by the first pass, left alone by
                     // the others (every gather is done: the next copies may go)
                     if (p == 0) {
@@ -539,7 +597,7 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
                             *reinterpret_cast<float2 *>(C.amp + 2 * (obase | L.o_col[j])) = make_float2(0.f, 0.f);
-                    } else if (tile + 1 < tiles) {
+                    } else if (tile + GROUPS < tiles) {
                         D::copy_tile<1>(C.amp, tnext, L, stage, g_t, cs_t);
                     }
                     tbase = tnext;
@@ -548,28 +606,28 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                 D::split_store<1>(tlane, y, 0u);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncthreads();
-                if (tid == 0) D::issue_ts(tgrp + 64, tgrp, smem_u32(smem + kTmOffB), smem_u32(smem + kTmOffB + kB), mb);
-                if (p > 0 && L.nsub == 1 && tile + 1 < tiles) D::copy_tile<1>(C.amp, tnext, L, stage, g_t, cs_t);
+                D::group_bar<128>(bar);
+                if (ltid == 0) D::issue_ts(tgrp + 64, tgrp, smem_u32(smem + kTmOffB), smem_u32(smem + kTmOffB + kB), mb);
+                if (p > 0 && L.nsub == 1 && tile + GROUPS < tiles) D::copy_tile<1>(C.amp, tnext, L, stage, g_t, cs_t);
                 for (int b = 0; b < L.nsub; ++b) {
                     const bool ok = mbar_wait(mb, phase);
                     phase ^= 1;
-                    if (__syncthreads_or(!ok)) { failed = true; break; }
+                    if (D::group_bar_or<128>(bar, !ok)) { failed = true; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t dreg = (b & 1) ? 0u : 64u;                // this block's accumulator
                     D::tmem_ld32(tlane + dreg, y);
                     D::tmem_ld32(tlane + dreg + 32, y + 32);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (b + 1 < L.nsub) {
-                        D::exchange_through<1, kTmThreads>(y, stage, xw0, xr0, L.xw_col[0], L.xr_col[0], 0);
+                        D::exchange_through<1, 128>(y, stage, xw0, xr0, L.xw_col[0], L.xr_col[0], bar);
                         D::split_store<1>(tlane + dreg, y, 0u);              // the next block's A
                         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        __syncthreads();                                     // also: every exchange read is done
-                        if (tid == 0)
+                        D::group_bar<128>(bar);                              // also: every exchange read is done
+                        if (ltid == 0)
                             D::issue_ts(tgrp + (dreg ^ 64u), tgrp + dreg, smem_u32(smem + kTmOffB + 2 * kB),
                                         smem_u32(smem + kTmOffB + 3 * kB), mb);
-                        if (p > 0 && tile + 1 < tiles) D::copy_tile<1>(C.amp, tnext, L, stage, g_t, cs_t);
+                        if (p > 0 && tile + GROUPS < tiles) D::copy_tile<1>(C.amp, tnext, L, stage, g_t, cs_t);
                     } else {
                         const uint64_t obase = tbase | orow;
                         if (L.vec_out) {
@@ -584,21 +642,7 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                                     make_float2(y[2 * j], y[2 * j + 1]);
                         }
                         acc_out += (double)D::sum_squares(y);
-                        if (last_pass) {
-                            float zt[kMaxZZ];
-#pragma unroll
-                            for (int i = 0; i < kMaxZZ; ++i) zt[i] = 0.f;
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                const uint64_t g = obase | L.o_col[j];
-                                const float pr = fmaf(y[2 * j], y[2 * j], y[2 * j + 1] * y[2 * j + 1]);
-                                const uint32_t par = (uint32_t)(g ^ (g >> 1));       // bit i: x_i xor x_{i+1}
-#pragma unroll
-                                for (int i = 0; i < kMaxZZ; ++i) zt[i] += ((par >> i) & 1u) ? -pr : pr;
-                            }
-#pragma unroll
-                            for (int i = 0; i < kMaxZZ; ++i) zz[i] += (double)zt[i];
-                        }
+                        if (last_pass) add_zz(zz, y, obase, L, nzz);
                     }
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 }
@@ -606,12 +650,14 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                 tbase = tnext;
             }
             asm volatile("cp.async.wait_group 0;" ::: "memory");
+            failed = __syncthreads_or(failed);
             // the pass's output norm (fixed order), and the next pass's scale
             for (int o = 16; o > 0; o >>= 1) acc_out += __shfl_xor_sync(0xffffffffu, acc_out, o);
-            __syncthreads();
             if (lane == 0) red[warp] = acc_out;
             __syncthreads();
-            out_norm = red[0] + red[1] + red[2] + red[3];
+            out_norm = red[0];
+#pragma unroll
+            for (int w = 1; w < kWarps; ++w) out_norm += red[w];
             scale = out_norm > 0 ? (float)(1.0 / sqrt(out_norm)) : 1.0f;
             // this pass's stores must be visible to the next pass's loads
             __threadfence();
@@ -625,10 +671,12 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
                 for (int o = 16; o > 0; o >>= 1) zz[i] += __shfl_xor_sync(0xffffffffu, zz[i], o);
             if (lane == 0)
 #pragma unroll
-                for (int i = 0; i < kMaxZZ; ++i) red[4 + warp * kMaxZZ + i] = zz[i];
+                for (int i = 0; i < kMaxZZ; ++i) red[kWarps + warp * kMaxZZ + i] = zz[i];
             __syncthreads();
             for (int i = tid; i < nzz; i += kTmThreads) {
-                const double sum = red[4 + i] + red[4 + kMaxZZ + i] + red[4 + 2 * kMaxZZ + i] + red[4 + 3 * kMaxZZ + i];
+                double sum = red[kWarps + i];
+#pragma unroll
+                for (int w = 1; w < kWarps; ++w) sum += red[kWarps + w * kMaxZZ + i];
                 if (shared) C.zzp[(size_t)task.part * kMaxZZ + i] = sum;
                 else C.zz[i] = sum / out_norm;
             }
@@ -642,7 +690,7 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
             if (*s_circ == C.npass * C.nparts) {             // the circuit's last part: its <ZZ>
                 __threadfence();
                 const double norm = sum_parts(C.norms + (size_t)task.pass * C.nparts, 1, C.nparts);
-                for (int i = warp; i < nzz; i += kTmThreads / 32) {
+                for (int i = warp; i < nzz; i += kWarps) {
                     const double sum = sum_parts(C.zzp + i, kMaxZZ, C.nparts);
                     if (lane == 0) C.zz[i] = sum / norm;
                 }
@@ -652,13 +700,13 @@ __global__ void __launch_bounds__(kTmThreads, kTmCtasPerSm) k_batch_tmem(BatchPa
     }
     if (failed) {
         if (tid == 0) atomicExch(P.err, 1);
-        mbar_wait(mb, phase ^ 1);
+        mbar_wait(mb, phase ^ 1);                            // bounded: the group's MMAs in flight, if any
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tgrp), "r"(kTmCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTmCols));
     }
 }
 
@@ -684,6 +732,7 @@ struct qs_batch {
     void *d_tasks = nullptr;             // BatchTask[ntasks] (k_batch_tmem)
     double *d_parts = nullptr;           // shared circuits' norms and <ZZ> sums
     int32_t ntasks = 0, nshared = 0;
+    int groups = 1;                      // lane groups per CTA of k_batch_tmem
     double *d_zz = nullptr;
     int32_t *d_head = nullptr;           // queue head, error flag, the shared circuits' counters
     size_t zz_count = 0, state_bytes = 0;
@@ -716,7 +765,37 @@ std::string signature(int nq, const qs_gate *g, size_t count)
     return s;
 }
 
-// The queue of k_batch_tmem for `ctas` resident CTAs.  A circuit is shared
+int tm_ctas(int groups)
+{
+    return QS_SM_COUNT * (groups == 2 ? TmShape<2>::kCtasPerSm : TmShape<1>::kCtasPerSm);
+}
+
+// Lane groups per CTA.  Two CTAs of two groups per SM have four tiles in flight
+// where three CTAs of one have three, but hold fewer circuits, and one of a
+// single tile keeps half of its CTA idle.  Two groups are taken
+//  - for up to 296 circuits (a CTA each) unless those of one tile are three
+//    quarters of the work (256 of 14 qubits: 0.27 -> 0.25 ms, of 10..13: 0.21
+//    -> 0.19; of 11 and 12: 0.137 with one group, 0.155 with two);
+//  - for more when the shared circuits of 32 tiles and up are most of it (400
+//    of 10..22 qubits: 14.6 -> 13.2 ms), or from three rounds of CTAs on those
+//    of 16 tiles (1024 of 10..20: 9.2 -> 8.3 ms; 600 of 17, two rounds: 3.4
+//    with one group, 3.9 with two; 1024 of 10..14: 0.46 and 0.57).
+int tm_groups(const std::vector<BatchCirc> &hc)
+{
+    const int ctas = tm_ctas(2);
+    auto work = [](const BatchCirc &c) { return (int64_t)c.npass << (c.nq_eff - 12); };
+    int64_t total = 0, one = 0, wide = 0, shared = 0;
+    for (const BatchCirc &c : hc) total += work(c);
+    for (const BatchCirc &c : hc) {
+        if (c.nq_eff == 12) one += work(c);
+        if (c.nq_eff >= 16) wide += work(c);
+        if (c.nq_eff >= 17 && 2 * ctas * work(c) > total) shared += work(c);
+    }
+    if (hc.size() <= (size_t)ctas) return 4 * one < 3 * total ? 2 : 1;
+    return 2 * shared > total || (hc.size() >= 3 * (size_t)ctas && 2 * wide > total) ? 2 : 1;
+}
+
+// The queue of k_batch_tmem for `ctas` resident CTAs of `groups` lane groups.  A circuit is shared
 // when alone it would take more than half of an even share of the work (in
 // tiles x passes): below that, longest-first over whole circuits ends within
 // that half.  All shared circuits run in step, by the passes they have left
@@ -725,7 +804,7 @@ std::string signature(int nq, const qs_gate *g, size_t count)
 // parts than CTAs, the rest follow.  A part costs its block matrices' load
 // once more (32 KB from L2), so it has at least 2 tiles.  Returns the doubles
 // that the shared circuits need; their norms / zzp get offsets into them.
-size_t plan_tasks(std::vector<BatchCirc> &hc, const std::vector<int32_t> &order, int ctas,
+size_t plan_tasks(std::vector<BatchCirc> &hc, const std::vector<int32_t> &order, int ctas, int groups,
                   std::vector<BatchTask> *tasks, int32_t *nshared)
 {
     auto tiles = [&](const BatchCirc &c) { return (int64_t)1 << (c.nq_eff - 12); };
@@ -744,12 +823,14 @@ size_t plan_tasks(std::vector<BatchCirc> &hc, const std::vector<int32_t> &order,
         }
     }
     const int64_t per = shared_tiles < 8 * (int64_t)ctas ? ctas : 2 * (int64_t)ctas;
-    const int32_t part = (int32_t)std::max<int64_t>(2, (shared_tiles + per - 1) / per);
+    const int32_t part = (int32_t)std::max<int64_t>(2, (shared_tiles + per * groups - 1) / (per * groups) * groups);
     size_t doubles = 0;
     for (int32_t i : shared) {
         BatchCirc &c = hc[(size_t)i];
-        c.part = part;
         c.nparts = (int32_t)((tiles(c) + part - 1) / part);
+        // even parts (8 tiles in 6 and 2: 400 circuits of 15 qubits lost a third)
+        const int32_t even = (int32_t)((tiles(c) + c.nparts - 1) / c.nparts);
+        c.part = (even + groups - 1) / groups * groups;
         c.norms = reinterpret_cast<double *>(doubles);
         doubles += (size_t)c.npass * c.nparts;
         c.zzp = reinterpret_cast<double *>(doubles);
@@ -1031,7 +1112,8 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
             });
         std::vector<BatchTask> tasks;
         if (B->use_tmem) {
-            const size_t doubles = plan_tasks(hc, B->order, QS_SM_COUNT * kTmCtasPerSm, &tasks, &B->nshared);
+            B->groups = tm_groups(hc);
+            const size_t doubles = plan_tasks(hc, B->order, tm_ctas(B->groups), B->groups, &tasks, &B->nshared);
             B->ntasks = (int32_t)tasks.size();
             e = cudaMalloc((void **)&B->d_parts, std::max<size_t>(doubles, 1) * sizeof(double));
             if (e == cudaSuccess) e = cudaMalloc(&B->d_tasks, std::max<size_t>(tasks.size(), 1) * sizeof(BatchTask));
@@ -1071,8 +1153,9 @@ int batch_launch(qs_batch *B, cudaStream_t st)
     P.head = B->d_head;
     P.err = B->d_head + 1;
     if (B->use_tmem) {
-        const unsigned grid = (unsigned)std::min(B->ntasks, QS_SM_COUNT * kTmCtasPerSm);
-        k_batch_tmem<<<grid, kTmThreads, kTmSmemBytes, st>>>(P);
+        const unsigned grid = (unsigned)std::min(B->ntasks, tm_ctas(B->groups));
+        if (B->groups == 2) k_batch_tmem<2><<<grid, TmShape<2>::kThreads, TmShape<2>::kSmemBytes, st>>>(P);
+        else k_batch_tmem<1><<<grid, TmShape<1>::kThreads, TmShape<1>::kSmemBytes, st>>>(P);
     } else if (B->opts.max_sub <= 2) {
         const unsigned grid = (unsigned)std::min(B->n, QS_SM_COUNT * BShape<2>::kCtasPerSm);
         k_batch<2><<<grid, kThreads, BShape<2>::kSmemBytes, st>>>(P);
@@ -1092,7 +1175,8 @@ extern "C" int qs_batch_run(qs_batch *B, void *stream)
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     QS_CUDA_TRY(cudaFuncSetAttribute(k_batch<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, BShape<2>::kSmemBytes));
     QS_CUDA_TRY(cudaFuncSetAttribute(k_batch<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, BShape<3>::kSmemBytes));
-    QS_CUDA_TRY(cudaFuncSetAttribute(k_batch_tmem, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmSmemBytes));
+    QS_CUDA_TRY(cudaFuncSetAttribute(k_batch_tmem<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TmShape<1>::kSmemBytes));
+    QS_CUDA_TRY(cudaFuncSetAttribute(k_batch_tmem<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TmShape<2>::kSmemBytes));
     if (!B->opts.use_graph) return batch_launch(B, st);
     if (!B->graph_exec) {
         // capture once on a private stream; replay on the caller's stream

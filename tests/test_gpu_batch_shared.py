@@ -33,3 +33,17 @@ def test_shared_circuits_match_oracle(need_gpu, name, order):
         ref_zz, ref_state = oracle_zz(q, g)
         assert np.abs(zz[k] - ref_zz).max() < TOL, (k, q)
         assert np.abs(b.state(k) - ref_state).max() < TOL, (k, q)
+
+
+@pytest.mark.parametrize("count,width", [(296, 13), (297, 13), (64, 12), (888, 16)])
+def test_lane_groups_match_oracle(need_gpu, count, width):
+    """Both sides of the rule for lane groups per CTA: circuits of one, two and
+    16 tiles, up to and past one circuit per CTA, one odd width among them."""
+    few = [(width, circuits.vqe_ansatz(width, 1 + k, seed=7 * width + k)) for k in range(2)]
+    few.append((width + 1, circuits.vqe_ansatz(width + 1, 2, seed=5)))
+    refs = [oracle_zz(q, g)[0] for q, g in few]
+    b = Batch([few[k % 2] for k in range(count - 1)] + [few[2]])
+    b.run()
+    zz = b.zz()
+    for k in range(count):
+        assert np.abs(zz[k] - refs[2 if k == count - 1 else k % 2]).max() < TOL, k
