@@ -1407,8 +1407,8 @@ def run_kernels(args):
     qs = np.arange(n, dtype=np.int32)
     u = np.random.default_rng(1).uniform(size=(SHOTS, n))
     timed("qs_sample: marginal + fold + k_shots, 1024 shots of all qubits", lambda: sv.sample(qs, u), S * N, calls=2)
-    timed("qs_prob_zero: k_half_sum + k_finalize (qubit 5)", lambda: sv.prob_zero(5), S * N // 2)
-    timed("qs_measure: k_half_sum + k_finalize + k_collapse (qubit 6)", lambda: sv.measure(6, 0.5),
+    timed("qs_prob_zero: k_half_sum (qubit 5)", lambda: sv.prob_zero(5), S * N // 2)
+    timed("qs_measure: k_half_sum + k_collapse (qubit 6)", lambda: sv.measure(6, 0.5),
           S * N // 2 + S * N + S * N // 2, calls=2)
     amp = C.c_void_p()
     check(L.qs_device_ptr(h, C.byref(amp)))
