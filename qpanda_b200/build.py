@@ -34,10 +34,7 @@ def _newer(src_list, target):
 
 
 CXX = os.environ.get("CXX_HOST", "g++")
-CXX# Jump tables for switches: nvcc's default makes them trees of compares, 7 deep
-# for k_stage's choice among an op's 80 kinds (10 compares and 10 branches an
-# op; 30-qubit depth-16 complex64 circuit 121.0 ms, with the table 113.0).
-FLAGS = ["-O3", "-std=c++17", "-fPIC", "-Wall", "-I" + os.path.join(ROOT, "include"),
+CXXFLAGS = ["-O3", "-std=c++17", "-fPIC", "-Wall", "-I" + os.path.join(ROOT, "include"),
             "-I/usr/local/cuda/include"]
 
 
