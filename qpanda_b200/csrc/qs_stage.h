@@ -546,7 +546,7 @@ QS_UNROLL
     case K_EX + 3: op_exchange<T, RB, 0, 3>(v, m, creg); break;
     case K_EX + 4: op_exchange<T, RB, 1, 3>(v, m, creg); break;
     case K_EX + 5: op_exchange<T, RB, 2, 3>(v, m, creg); break;
-    default: break;
+    default: __builtin_unreachable();      // no range check before the jump table
     }
 }
 
