@@ -459,8 +459,8 @@ def run_b200(args):
                                         else circuits.gate_bytes(gates, n, amp_b)) / ot / 1e9,
                   "dominant_kernel": odom, "dominant_gbs": o_ach, "dominant_frac": o_ach / peak,
                   "kernels": kernel_table(okinds)}
-    # the plain path as a caller gets it: qs_gates_apply, whose runs of gates
-    # on one tile's qubits go through shared memory in one pass each
+    # the plain path as a caller gets it: qs_gates_apply, many gates
+    # per read and write of the state (staged passes)
     staged_s = None
     if other == "plain" or path == "plain":
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -474,8 +474,8 @@ def run_b200(args):
             other_line["circuit_s_per_gate_launches"] = ot
             other_line["circuit_s"] = ot = staged_s
             other_line["hbm_gbs_effective"] = circuits.gate_bytes(gates, n, amp_b) / ot / 1e9
-            other_line["note"] = ("circuit_s: qs_gates_apply (runs of consecutive gates whose targets share "
-                                  "one tile's 10 qubits staged in shared memory and registers, one pass each); "
+            other_line["note"] = ("circuit_s: qs_gates_apply (staged passes: tiles of 12 qubits in registers, "
+                                  "many gates per read and write of the state); "
                                   "kernels: the same gates one launch each")
 
     # fidelity of the fused complex64 run against the complex128 per-gate path
@@ -1226,8 +1226,8 @@ def qft_line(args, n, steps, warmup, gpu_id=None):
             table[kind_of[op]] = {"launches_per_circuit": len(ts) // steps, "mean_ms": t * 1e3,
                                   "gbs": gbs, "frac": gbs / peak}
         cs = statistics.mean(circ)
-        # the same gates through qs_gates_apply: runs of gates that share one
-        # tile's qubits staged, one pass each (the state it leaves is the one above)
+        # the same gates through qs_gates_apply: staged passes, many
+        # gates each (the state it leaves is the one above up to rounding)
         staged = []
         for k in range(warmup + steps):
             sv.set_state(host)
@@ -1242,7 +1242,7 @@ def qft_line(args, n, steps, warmup, gpu_id=None):
         ss = statistics.mean(staged)
         out[dt] = {"circuit_s": cs, "hbm_gbs_effective": circuits.gate_bytes(gates, n, amp_b) / cs / 1e9,
                    "kernels": table, "staged_circuit_s": ss,
-                   "staged_note": "qs_gates_apply: runs of consecutive gates whose targets share one tile's 10 qubits, one staged pass each"}
+                   "staged_note": "qs_gates_apply: staged passes on tiles of 12 qubits, many gates each"}
         states[dt] = sv
     clk = clocks.stop() if clocks else None
     a, d = states["c64"], states["c128"]
@@ -1389,10 +1389,10 @@ def run_kernels(args):
     timed("k_quad: 4x4 on (3, 17)", lambda: check(L.qs_apply_2q(h, 3, 17, m2.ctypes.data_as(C.POINTER(C.c_double)),
                                                                  0)), 2 * S * N)
     run = circuits.make_gates([("RY", (q,), 0.2 * q) for q in range(10)])
-    timed("k_lowstage: 10 rotations on qubits 0..9 (one pass)",
+    timed("k_stage: 10 rotations on qubits 0..9 (one pass)",
           lambda: check(L.qs_gates_apply(h, C.c_void_p(run.ctypes.data), len(run))), 2 * S * N)
     run_hi = circuits.make_gates([("RY", (q,), 0.2 * q) for q in range(n - 7, n)])
-    timed(f"k_lowstage: 7 rotations on qubits {n - 7}..{n - 1} (one pass; tile qubits 0..2 and {n - 7}..{n - 1})",
+    timed(f"k_stage: 7 rotations on qubits {n - 7}..{n - 1} (one pass)",
           lambda: check(L.qs_gates_apply(h, C.c_void_p(run_hi.ctypes.data), len(run_hi))), 2 * S * N)
     qs20 = np.arange(20, dtype=np.int32)
     dev = torch.empty(1 << 20, dtype=torch.float64, device="cuda")

@@ -124,7 +124,8 @@ int qs_get_state(qs_state *s, void *host_out, int host_dtype);
  * reference leaves as no-ops (:914-922, :1054-1062), act on the control=1
  * subspace here. */
 int qs_gate_apply(qs_state *s, const qs_gate *g);
-/* Apply count gate records in order (one launch per gate, no fusion). */
+/* Apply count gate records: the state is as if they were applied in order, up
+ * to rounding (many gates per pass over the state on 8 qubits and more). */
 int qs_gates_apply(qs_state *s, const qs_gate *g, size_t count);
 
 /* ---- generic unitaries (the kernels the gate records lower to) --------- */
