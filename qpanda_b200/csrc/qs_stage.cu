@@ -274,9 +274,12 @@ int apply_t(qs_state *s, const std::vector<qs_prim> &prims)
         for (int i : pass) traffic += op_traffic(P, P.ops[(size_t)i]);
         int r = QS_OK;
         const bool zeros = finite && (s->untouched & ~qmask) != 0;
-        if (pass.size() == 1 || (traffic <= 1.0 && s->amp_bytes() >= (64ull << 20))) {
+        auto one_by_one = [&]() {
             for (size_t k = 0; !r && k < pass.size(); ++k) r = launch_op(s, P, P.ops[(size_t)pass[k]]);
-            if (r) return r;
+            return r;
+        };
+        if (pass.size() == 1 || (traffic <= 1.0 && s->amp_bytes() >= (64ull << 20))) {
+            if (one_by_one()) return r;
             continue;
         }
         bool done = false;
@@ -288,6 +291,10 @@ int apply_t(qs_state *s, const std::vector<qs_prim> &prims)
         }
         if (!done) {
             plan_pass<RunLarge<T>, T>(P, qmask, pass, &large, &rest);
+            if (rest.size() == pass.size()) {        // none fits a parameter block: planned again, none would
+                if (one_by_one()) return r;
+                continue;
+            }
             if (!rest.empty()) P.give_back(rest);
             large.zeros = zeros;
             r = launch<T>(s, large);

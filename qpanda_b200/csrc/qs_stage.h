@@ -146,6 +146,7 @@ struct Run {
 template <typename T> using RunSmall = Run<T, 40, 12, 2, 24>;
 template <typename T> using RunLarge = Run<T, 208, 56, 16, 256>;
 static_assert(sizeof(RunLarge<double>) <= 32764, "kernel parameters are at most 32764 bytes");
+static_assert(RunLarge<double>::NENT > 64, "a ladder has a term per qubit and one on its hub alone: any one fits");
 
 // ------------------------------------------------------------------ index maps
 // the weight of tile bit b in shared-memory slots: digit d of base 2^LB

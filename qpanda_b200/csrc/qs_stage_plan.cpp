@@ -112,7 +112,9 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
         if (p.kind == QS_PRIM_PHASE) {
             if (last_diag >= 0 && !(since & p.holes)) {
                 // join the last phase op when every term then has at most one
-                // qubit beside a common hub
+                // qubit beside a common hub; phases on one qubit are one term, so
+                // that a ladder has at most one per qubit and fits a parameter block
+                // however many phases share its hub
                 GOp &d = ops[last_diag];
                 const uint64_t hub = d.ctrl & p.holes;
                 const uint64_t mine = p.holes & ~hub, first = d.ctrl & ~hub;
@@ -121,8 +123,16 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
                     if (first) terms[d.first].q = low_bit(first);
                     d.ctrl = hub;
                     d.diag |= p.holes;
-                    terms.push_back({mine ? low_bit(mine) : -1, p.m[0], p.m[1]});
-                    ++d.count;
+                    const int q = mine ? low_bit(mine) : -1;
+                    auto t = std::find_if(terms.begin() + d.first, terms.end(), [&](const Term &x) { return x.q == q; });
+                    if (t == terms.end()) {
+                        terms.push_back({q, p.m[0], p.m[1]});
+                        ++d.count;
+                    } else {
+                        const cd w = cd(t->re, t->im) * cd(p.m[0], p.m[1]);
+                        t->re = w.real();
+                        t->im = w.imag();
+                    }
                     continue;
                 }
             }
@@ -657,9 +667,8 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
                     if (!out_q && reg_of[pos[t.q]] >= 0) {
                         if (side) continue;
                         T *w = &op.m[2 * reg_of[pos[t.q]]];
-                        const cd z = cd(t.re, t.im) * cd((double)w[0], (double)w[1]);
-                        w[0] = (T)z.real();
-                        w[1] = (T)z.imag();
+                        w[0] = (T)t.re;
+                        w[1] = (T)t.im;
                     } else if (out_q == (side == 1)) {
                         S.ent[nent++] = {t.re, t.im, alone ? -1 : out_q ? t.q : thread_of[pos[t.q]], 0};
                         ++(out_q ? L.nout : L.nthr);

@@ -7,9 +7,9 @@ import numpy as np
 import pytest
 
 from oracle.pyoracle import OracleState
-from qpanda_b200 import StateVector, circuits
+from qpanda_b200 import Server, StateVector, circuits
 from qpanda_b200.capi import check, lib
-from tests.test_stage_emulation import LISTS, swaps
+from tests.test_stage_emulation import LISTS, MANY_PHASES, swaps
 
 pytestmark = pytest.mark.gpu
 
@@ -99,3 +99,32 @@ def test_closing_exchange(need_gpu, kind, n, dtype):
     o.set_state(init)
     o.apply(gates)
     assert np.abs(got - o.state()).max() < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("kind", list(MANY_PHASES))
+def test_many_phases_on_one_hub(need_gpu, kind, dtype):
+    n, gates = MANY_PHASES[kind][0], MANY_PHASES[kind][1]()
+    init = random_state(n, n)
+    with StateVector(n, dtype) as sv:
+        sv.set_state(init.astype(np.complex64) if dtype == "c64" else init)
+        sv.apply(gates)
+        got = sv.get_state()
+    o = OracleState(n)
+    o.set_state(init)
+    o.apply(gates)
+    # FP64: two roundings of 1.1e-16 per gate on either side
+    assert np.abs(got - o.state()).max() < max(TOL[dtype], 4.5e-16 * len(gates))
+
+
+def test_many_phases_on_one_hub_served(need_gpu):
+    """The same through the serving loop, below the width of its plans."""
+    n, gates = MANY_PHASES["estimation10"][0], MANY_PHASES["estimation10"][1]()
+    srv = Server(slots=1)
+    rid = srv.submit(n, gates, "probs")
+    srv.wait(rid)
+    o = OracleState(n)
+    o.apply(gates)
+    assert np.abs(srv.fetch_probs(rid) - o.probs()).max() < 1e-5
+    srv.release(rid)
+    srv.close()

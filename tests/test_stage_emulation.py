@@ -130,3 +130,52 @@ def test_closing_exchange_matches_oracle(emu, kind, n, dtype):
 ])
 def test_benchmark_circuits_run_in_few_passes(emu, n, gates, dtype, most):
     assert plan(emu, n, gates(), dtype)[0] <= most
+
+
+def phase_estimation(n):
+    """Phase estimation of a phase gate on the highest qubit with n - 1 counting
+    qubits, textbook form: 2^k controlled phases from counting qubit k, so that
+    2^(n-1) - 1 phases share a hub, then the inverse QFT of the counting qubits."""
+    t = n - 1
+    spec = [("X", (t,))] + [("H", (k,)) for k in range(t)]
+    spec += [("CR", (k, t), 0.7) for k in range(t) for _ in range(1 << k)]
+    for j in reversed(range(t)):
+        spec += [("H", (j,))] + [("CR", (j, i), -np.pi / 2 ** (j - i)) for i in range(j)]
+    return circuits.make_gates(spec)
+
+
+def phases_on(n, hubs, count):
+    """`count` phases on each hub, the partners in turn, then an H on it."""
+    spec = []
+    for h in hubs:
+        others = [q for q in range(n) if q != h]
+        spec += [("CR", (h, others[k % len(others)]), 0.1 + 0.01 * k) for k in range(count)] + [("H", (h,))]
+    return circuits.make_gates(spec)
+
+
+# lists whose phases on one hub outnumber a parameter block's entries
+MANY_PHASES = {
+    "estimation10": (10, lambda: phase_estimation(10)),
+    "estimation13": (13, lambda: phase_estimation(13)),
+    "hub300": (12, lambda: phases_on(12, [0], 300)),
+    "hub257": (10, lambda: phases_on(10, [0], 257)),
+    "hubs": (13, lambda: phases_on(13, [0, 12, 5], 300)),
+    "pair300": (9, lambda: circuits.make_gates([("CR", (2, 7), 0.3 + 0.01 * k) for k in range(300)] + [("H", (2,)), ("H", (7,))])),
+}
+
+
+@pytest.mark.parametrize("dtype", [C64, C128])
+@pytest.mark.parametrize("kind", list(MANY_PHASES))
+def test_many_phases_on_one_hub(emu, kind, dtype):
+    n, gates = MANY_PHASES[kind][0], MANY_PHASES[kind][1]()
+    rng = np.random.default_rng(n)
+    init = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    init /= np.linalg.norm(init)
+    st = init.copy()
+    plan(emu, n, gates, dtype, st)
+    o = OracleState(n)
+    o.set_state(init)
+    o.apply(gates)
+    # FP64: two roundings of 1.1e-16 per gate on either side; FP32: phases on a
+    # hub are multiplied in FP64, so that their number does not show
+    assert np.abs(st - o.state()).max() < (TOL[C64] if dtype == C64 else 4.5e-16 * len(gates))
