@@ -195,25 +195,44 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
     }
     left.reserve(ops.size());
     for (size_t i = 0; i < ops.size(); ++i)
-        if (ops[i].type != G_NONE) left.push_back((int)i);
+        if (ops[i].type != G_NONE) left.push_back({ops[i].tgt, ops[i].diag, (int)i});
 }
 
-// The ops of list that can run in a pass on the tile of q: their targets in
-// q, and they commute with every earlier op that stays behind.  Returns their
-// number; *wants gets the target sets that alone keep an op out, *kept the
-// ops that stay behind (the rest of the list from where nothing can run).
-int Planner::scan(const std::vector<Masks> &list, uint64_t q, std::vector<uint64_t> *wants,
-                  std::vector<Masks> *kept) const
+// The ops left that can run in a pass on the tile of q: their targets in q, and
+// they commute with every earlier op that stays behind.  A scan looks at kWindow
+// ops at most, and no further than where nothing can run.  count() returns how
+// many there are; take() moves them into *taken (up to kPassOps), and *wants, if
+// asked for, gets the target sets that alone keep an op out.
+int Planner::count(uint64_t q) const
 {
     const uint64_t all = n >= 64 ? ~0ull : (1ull << n) - 1;
     uint64_t skip_all = 0, skip_tgt = 0;
-    int count = 0;
-    const size_t size = list.size();
-    for (size_t i = 0; i < size; ++i) {
-        const Masks &g = list[i];
+    int found = 0;
+    const Masks *g = left.data() + front, *const end = g + std::min(left.size() - front, kWindow);
+    for (; g < end; ++g) {
+        if (!(g->tgt & (skip_all | ~q)) && !(g->diag & skip_tgt)) {
+            ++found;
+            continue;
+        }
+        skip_all |= g->tgt | g->diag;
+        skip_tgt |= g->tgt;
+        if ((skip_all & all) == all) break;
+    }
+    return found;
+}
+
+void Planner::take(uint64_t q, std::vector<uint64_t> *wants, std::vector<int> *taken)
+{
+    const uint64_t all = n >= 64 ? ~0ull : (1ull << n) - 1;
+    uint64_t skip_all = 0, skip_tgt = 0;
+    behind.clear();
+    Masks *const from = left.data() + front, *const end = from + std::min(left.size() - front, kWindow);
+    Masks *p = from;
+    for (; p < end && (skip_all & all) != all && taken->size() < kPassOps; ++p) {
+        const Masks g = *p;
         const bool free = !(g.tgt & skip_all) && !(g.diag & skip_tgt);
         if (free && !(g.tgt & ~q)) {
-            ++count;
+            taken->push_back(g.op);
             continue;
         }
         if (free && wants) {
@@ -222,34 +241,26 @@ int Planner::scan(const std::vector<Masks> &list, uint64_t q, std::vector<uint64
         }
         skip_all |= g.tgt | g.diag;
         skip_tgt |= g.tgt;
-        if (kept) kept->push_back(g);
-        if ((skip_all & all) == all) {
-            if (kept) kept->insert(kept->end(), list.begin() + (long)i + 1, list.end());
-            break;
-        }
+        behind.push_back(g);
     }
-    return count;
+    // what was passed over moves up to where the scan stopped
+    std::copy(behind.begin(), behind.end(), p - behind.size());
+    front += (size_t)(p - from) - behind.size();
 }
 
 bool Planner::next(uint64_t *qmask, std::vector<int> *pass_ops)
 {
     pass_ops->clear();
-    if (left.empty()) return false;
+    if (front == left.size()) return false;
     uint64_t q = n <= K ? (1ull << n) - 1 : (1ull << low) - 1;
-    // the ops that stay behind so far: what runs on a tile runs on every
-    // larger one, so a round looks at the rest only
-    std::vector<Masks> rest, behind;
-    rest.reserve(left.size());
-    for (int i : left) rest.push_back({ops[(size_t)i].tgt, ops[(size_t)i].diag, i});
-    behind.reserve(left.size());
     std::vector<uint64_t> wants;
     double last[64];                               // a qubit's gain when it was last looked at
     for (double &g : last) g = 1e9;
     while (true) {
+        // what runs on a tile runs on every larger one, so a round looks at what
+        // stays behind only
         wants.clear();
-        behind.clear();
-        scan(rest, q, popc(q) < K ? &wants : nullptr, &behind);
-        rest.swap(behind);
+        take(q, popc(q) < K ? &wants : nullptr, pass_ops);
         if (popc(q) >= K) break;
         // grow the tile by the target set that lets the most ops per qubit in;
         // gains change little from round to round, so sets are looked at by
@@ -260,7 +271,7 @@ bool Planner::next(uint64_t *qmask, std::vector<int> *pass_ops)
         double best_gain = -1;
         for (uint64_t w : wants) {
             if (guess(w) < best_gain * 0.5) break;
-            const double gain = (double)scan(rest, q | w, nullptr, nullptr) / popc(w);
+            const double gain = (double)count(q | w) / popc(w);
             if (popc(w) == 1) last[low_bit(w)] = gain;
             if (gain > best_gain) {
                 best_gain = gain;
@@ -273,27 +284,26 @@ bool Planner::next(uint64_t *qmask, std::vector<int> *pass_ops)
         }
         for (int b = 0; b < n && popc(q) < K; ++b) q |= 1ull << b;
     }
-    // the pass: what did not stay behind (both ascending)
-    size_t k = 0, o = 0;
-    for (size_t i = 0; i < left.size(); ++i) {
-        if (k < rest.size() && left[i] == rest[k].op) {
-            ++k;
-            left[o++] = left[i];
-        } else {
-            pass_ops->push_back(left[i]);
-        }
-    }
-    left.resize(o);
+    std::sort(pass_ops->begin(), pass_ops->end());
     *qmask = q;
     return true;
 }
 
 void Planner::give_back(const std::vector<int> &rest)
 {
-    std::vector<int> all;
-    all.reserve(left.size() + rest.size());
-    std::merge(left.begin(), left.end(), rest.begin(), rest.end(), std::back_inserter(all));
-    left.swap(all);
+    if (rest.empty()) return;
+    // into the places that they and the pass's ops left free, in order
+    size_t end = front;
+    while (end < left.size() && left[end].op < rest.back()) ++end;
+    behind.assign(left.begin() + (long)front, left.begin() + (long)end);
+    front -= rest.size();
+    auto b = behind.begin();
+    auto out = left.begin() + (long)front;
+    for (int i : rest) {
+        while (b != behind.end() && b->op < i) *out++ = *b++;
+        *out++ = {ops[(size_t)i].tgt, ops[(size_t)i].diag, i};
+    }
+    std::copy(b, behind.end(), out);
 }
 
 namespace {
@@ -325,12 +335,13 @@ bool plan_permute(const Planner &plan, Permute *P)
     constexpr int RB = Traits<T>::RB, LOW = Traits<T>::LOW;
     constexpr int K = RB + 8;                          // 256 threads (128 when no bit is left without its partner)
     const int n = plan.n;
-    if (n < K || plan.left.size() < 2 || plan.left.size() > 16 + K / 2) return false;
+    const size_t left = plan.left.size() - plan.front;
+    if (n < K || left < 2 || left > 16 + K / 2) return false;
     int partner[64];
     for (int q = 0; q < n; ++q) partner[q] = q;
     uint64_t all = 0;
-    for (int i : plan.left) {
-        const GOp &g = plan.ops[(size_t)i];
+    for (size_t i = plan.front; i < plan.left.size(); ++i) {
+        const GOp &g = plan.ops[(size_t)plan.left[i].op];
         if (g.type != G_SWAP || (all & g.tgt)) return false;
         all |= g.tgt;
         const int a = low_bit(g.tgt), b = 63 - __builtin_clzll(g.tgt);

@@ -8,6 +8,7 @@ without renamed qubits must be free of bank conflicts.
 import ctypes as C
 import os
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -179,3 +180,45 @@ def test_many_phases_on_one_hub(emu, kind, dtype):
     # FP64: two roundings of 1.1e-16 per gate on either side; FP32: phases on a
     # hub are multiplied in FP64, so that their number does not show
     assert np.abs(st - o.state()).max() < (TOL[C64] if dtype == C64 else 4.5e-16 * len(gates))
+
+
+def idle(n, layers):
+    """Layers that leave the highest qubit alone until the last gate."""
+    return np.concatenate([circuits.random_layers(n - 1, layers, n), circuits.make_gates([("H", (n - 1,))])])
+
+
+@pytest.mark.parametrize("dtype", [C64, C128])
+@pytest.mark.parametrize("n", [9, 13])
+@pytest.mark.parametrize("kind", ["layers", "idle"])
+def test_lists_past_the_planning_window(emu, kind, n, dtype):
+    """More gates than the planner looks at at once and than a pass is handed."""
+    layers = 3000 // (n + n // 2)
+    gates = circuits.random_layers(n, layers, n) if kind == "layers" else idle(n, layers)
+    rng = np.random.default_rng(n)
+    init = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    init /= np.linalg.norm(init)
+    st = init.copy()
+    plan(emu, n, gates, dtype, st)
+    o = OracleState(n)
+    o.set_state(init)
+    o.apply(gates)
+    # as above: per gate two roundings on either side, FP32 as TOL for its 150 gates
+    assert np.abs(st - o.state()).max() < (TOL[C64] / 150 if dtype == C64 else 4.5e-16) * len(gates)
+
+
+@pytest.mark.parametrize("n,kind", [(9, "layers"), (12, "layers"), (20, "layers"), (20, "idle")])
+def test_planning_time_is_linear(emu, n, kind):
+    """Time per gate of 60,000 gates stays near that of 2,000 (copies of the
+    rest of the list in every pass made it ten times as long)."""
+    def per_gate(count):
+        layers = 2000 // (n + n // 2)
+        one = circuits.random_layers(n, layers, n) if kind == "layers" else idle(n, layers)
+        gates = np.tile(one, max(1, count // len(one)))
+        best = 1e9
+        for _ in range(3):
+            t = time.perf_counter()
+            plan(emu, n, gates, C64)
+            best = min(best, time.perf_counter() - t)
+        return best / len(gates)
+
+    assert per_gate(60000) < 3 * per_gate(2000)
