@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "qs_common.cuh"
+#include "qs_prim.h"
 
 namespace {
 
@@ -781,13 +782,14 @@ int measure_t(qs_state *s, int q, double u, int *outcome)
     return QS_OK;
 }
 
+constexpr size_t kMaxPartials = 32 << 20;
+
 // Marginal over qubits[0..m): plan the launch.  *part_bytes receives the
 // scratch the partial slices need (0 when one slice covers the space).
-MargParams marginal_plan(const qs_state *s, const int *qubits, int m, size_t *part_bytes)
+MargParams marginal_plan(int n, int dtype, const int *qubits, int m, size_t *part_bytes)
 {
     MargParams P;
     memset(&P, 0, sizeof(P));
-    const int n = s->n;
     P.c = n < 12 ? n : 12;
     P.m = m;
     uint64_t meas = 0;
@@ -802,26 +804,33 @@ MargParams marginal_plan(const qs_state *s, const int *qubits, int m, size_t *pa
         if (q < P.c) P.ulo_pos[P.ulo++] = q;
         else P.uhi_pos[P.uhi++] = q - P.c;
     }
-    // Aim for ~4 CTAs per SM in total.
     uint64_t ohi = 1ull << P.mhi, uspace = 1ull << P.uhi;
     P.uspace = uspace;
     uint64_t G = 1;
     if (P.c < 12) {
+        // aim for 4 CTAs per SM in total
         while (G < uspace && ohi * G < (uint64_t)QS_SM_COUNT * 4) G <<= 1;
     } else {
         // Slices are cut so that the CTAs of k_marginal_direct come out at whole
         // waves (as a power of two they came to 2.3 of 3, or 1.2 of 2).  Time of w
         // waves: their chunks at HBM rate, plus the slices' partials written,
         // read and added (in bytes per CTA slot, both sides at the same rate).
+        // One slice stays where that promises less than 5 %, which a launch and
+        // the partials' memory are not worth, and the partials take 32 MB at most:
+        // 20 low qubits of 27, complex64: one slice 197 us, the eight that are
+        // best by this model 230, with 64 MB of partials; of 28 360 and 390; of 30
+        // 1382 and 1343.
         const uint64_t slots = (uint64_t)QS_SM_COUNT * kMargCtas;
-        const double chunk = 4096.0 * (s->dtype == QS_C64 ? 8 : 16) * (double)slots;
-        double best = -1;
+        const double chunk = 4096.0 * (dtype == QS_C64 ? 8 : 16) * (double)slots;
+        auto time = [&](uint64_t g) {
+            const uint64_t waves = (ohi * g + slots - 1) / slots;
+            return (double)(waves * ((uspace + g - 1) / g)) * chunk + (g > 1 ? (2.0 * (double)g + 1) * (8ull << m) : 0);
+        };
+        double best = 0.95 * time(1);
         for (uint64_t w = 1; w <= 8; ++w) {
             const uint64_t g = std::min(uspace, std::max<uint64_t>(1, slots * w / ohi));
-            const uint64_t waves = (ohi * g + slots - 1) / slots;
-            const double t = (double)(waves * ((uspace + g - 1) / g)) * chunk + (g > 1 ? (2.0 * (double)g + 1) * (8ull << m) : 0);
-            if (best < 0 || t < best) {
-                best = t;
+            if (g * (8ull << m) <= kMaxPartials && time(g) < best) {
+                best = time(g);
                 G = g;
             }
         }
@@ -884,7 +893,7 @@ template <typename T>
 int probs_t(qs_state *s, const int *qubits, int m, double *out)
 {
     size_t outb = 8ull << m, part_b = 0;
-    MargParams P = marginal_plan(s, qubits, m, &part_b);
+    MargParams P = marginal_plan(s->n, s->dtype, qubits, m, &part_b);
     const size_t o_part = kBufOff + ((outb + 255) & ~255ull);
     int r = qs_ensure_scratch(s, o_part + part_b);
     if (r) return r;
@@ -902,19 +911,39 @@ int probs_t(qs_state *s, const int *qubits, int m, double *out)
     return QS_OK;
 }
 
+// Where a sampler call keeps what in scratch, and the marginal of its tree.
+struct SampleLayout {
+    int K0;                                       // levels of the tree
+    size_t u_b, out_b, o_tree, o_u, o_out, o_part, bytes;
+    MargParams marg;
+};
+
+SampleLayout sample_layout(int n, int dtype, const int *qubits, int m, size_t shots)
+{
+    SampleLayout L;
+    L.K0 = m < kTreeQubits ? m : kTreeQubits;
+    L.u_b = 8ull * shots * (size_t)m;
+    L.out_b = 8ull * shots;
+    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    L.o_tree = kBufOff;
+    L.o_u = L.o_tree + al(16ull << L.K0);         // 2^(K0+1) doubles
+    L.o_out = L.o_u + al(L.u_b);
+    L.o_part = L.o_out + al(L.out_b);
+    size_t part_b = 0;
+    L.marg = marginal_plan(n, dtype, qubits, L.K0, &part_b);
+    L.bytes = L.o_part + part_b;
+    return L;
+}
+
 template <typename T>
 int sample_t(qs_state *s, const int *qubits, int m, const double *u, size_t shots, uint64_t *out)
 {
-    const int K0 = m < kTreeQubits ? m : kTreeQubits;
-    const size_t tree_b = 16ull << K0;            // 2^(K0+1) doubles
-    const size_t u_b = 8ull * shots * (size_t)m;
-    const size_t out_b = 8ull * shots;
-    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    size_t o_tree = kBufOff, o_u = o_tree + al(tree_b), o_out = o_u + al(u_b), o_part = o_out + al(out_b);
-    size_t part_b = 0;
-    MargParams P = marginal_plan(s, qubits, K0, &part_b);
+    const SampleLayout L = sample_layout(s->n, s->dtype, qubits, m, shots);
+    const int K0 = L.K0;
+    const size_t u_b = L.u_b, out_b = L.out_b, o_tree = L.o_tree, o_u = L.o_u, o_out = L.o_out, o_part = L.o_part;
+    const MargParams &P = L.marg;
     // Size scratch once, before any pointer into it is taken.
-    int r = qs_ensure_scratch(s, o_part + part_b);
+    int r = qs_ensure_scratch(s, L.bytes);
     if (r) return r;
     char *sc = static_cast<char *>(s->scratch);
     ShotParams SP;
@@ -965,6 +994,12 @@ int sample_t(qs_state *s, const int *qubits, int m, const double *u, size_t shot
 }  // namespace
 
 // ------------------------------------------------------------------ C ABI
+// Scratch that qs_sample takes (before qs_ensure_scratch rounds it up to a power of two).
+extern "C" size_t qs_sample_scratch_bytes(int n, int dtype, const int *qubits, int m, size_t shots)
+{
+    return sample_layout(n, dtype, qubits, m, shots).bytes;
+}
+
 extern "C" int qs_prob_zero(qs_state *s, int q, double *p0)
 {
     int r = qs_check_state(s);
@@ -1000,7 +1035,7 @@ extern "C" int qs_probs_device(qs_state *s, const int *qubits, int m, double *de
     if ((r = check_qubit_list(s, qubits, m, "qs_probs_device"))) return r;
     if (!dev_out) return qs_fail(QS_ERR_ARG, "qs_probs_device: null output");
     size_t part_b = 0;
-    MargParams P = marginal_plan(s, qubits, m, &part_b);
+    MargParams P = marginal_plan(s->n, s->dtype, qubits, m, &part_b);
     if ((r = qs_ensure_scratch(s, kBufOff + part_b))) return r;
     double *part = reinterpret_cast<double *>(static_cast<char *>(s->scratch) + kBufOff);
     return s->dtype == QS_C64 ? marginal_launch<float>(s, P, dev_out, part)

@@ -19,6 +19,8 @@ struct qs_prim {
 // Lower one gate record on an n-qubit register; QS_OK or a QS_ERR_* code
 // (the message is recorded for qs_last_error()).
 int qs_lower_gate(int n, const qs_gate *g, qs_prim *p);
+// Scratch of a qs_sample call (qs_measure.cu), before it is rounded up to a power of two.
+extern "C" size_t qs_sample_scratch_bytes(int n, int dtype, const int *qubits, int m, size_t shots);
 // All qubits (targets and controls) a gate touches.
 uint64_t qs_gate_qubits(const qs_gate *g);
 

@@ -61,7 +61,7 @@ struct Request {
 size_t footprint_of(int n, int kind)
 {
     const size_t state = 8ull << n;                   // complex64
-    const size_t scratch = 64ull << 20;               // reductions, sampling tree, plan matrices
+    const size_t scratch = 64ull << 20;               // reductions, sampling tree (qs_sample_scratch_bytes: 1024 shots fit)
     return state + scratch + (kind == QS_REQ_PROBS ? (8ull << n) : 0);
 }
 
