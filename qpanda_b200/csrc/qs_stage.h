@@ -17,8 +17,8 @@
 //    where the product keeps their form, or three or more follow;
 //  - a real or RX-like 1-qubit matrix is taken as p * [[1, r], [q, +-1]] with
 //    its largest row entry p pulled out: 4 multiply-adds per amplitude pair
-//    instead of 16; the p's of a pass are collected (FP64, on the host) and
-//    applied once, when the tile is stored;
+//    instead of 16; the p's of a pass are collected (in extended precision, on the
+//    host) and applied once, when the tile is stored;
 //  - controlled phases that share a qubit (a QFT's CR ladder) become one
 //    diagonal factor per amplitude, a product of per-qubit phases;
 //  - a SWAP of two tile qubits renames tile bits and costs nothing;
@@ -583,6 +583,7 @@ struct GOp {
     uint64_t ctrl;               // G_CU, G_EX: controls; G_DIAG: the hub (bits every term shares)
     uint64_t off0, off1;         // G_EX: the exchanged qubits
     double m[8];                 // G_U, G_CU, G_EX: 2x2; G_DIAG: m[0] + i m[1] a factor of every amplitude
+    long double det;             // G_U: |det| of its gates, before their product was rounded
     int first, count;            // G_DIAG: its terms [first, first + count) in Planner::terms
 };
 struct Term {

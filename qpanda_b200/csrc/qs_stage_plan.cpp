@@ -10,6 +10,13 @@ namespace qs_stg {
 namespace {
 
 typedef std::complex<double> cd;
+typedef std::complex<long double> cl;
+
+// a * b without std::complex's look at infinities
+inline cl mul(const cl &a, const cl &b)
+{
+    return cl(a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real());
+}
 
 inline int popc(uint64_t x) { return __builtin_popcountll(x); }
 inline int low_bit(uint64_t x) { return __builtin_ctzll(x); }
@@ -28,6 +35,15 @@ int form(const double m[8])
     if (m[1] == 0 && m[3] == 0 && m[5] == 0 && m[7] == 0) return 1;
     if (m[1] == 0 && m[7] == 0 && m[2] == 0 && m[4] == 0) return 2;
     return 3;
+}
+
+// |det| of a 2x2 row-major complex matrix: how it scales the norm, squared
+template <typename T>
+long double abs_det(const T m[8])
+{
+    const long double re = (long double)m[0] * m[6] - (long double)m[1] * m[7] - (long double)m[2] * m[4] + (long double)m[3] * m[5];
+    const long double im = (long double)m[0] * m[7] + (long double)m[1] * m[6] - (long double)m[2] * m[5] - (long double)m[3] * m[4];
+    return im == 0 ? std::fabs(re) : std::sqrt(re * re + im * im);
 }
 
 // a := b * a, 2x2 row-major complex
@@ -85,12 +101,14 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
             const int o = open[q];
             if (o >= 0 && (form(ops[o].m) == form(p.m) || form(ops[o].m) == 3)) {
                 mul2(ops[o].m, p.m);
+                ops[o].det *= abs_det(p.m);
                 continue;
             }
             if (o >= 0 && before[q] >= 0) {
                 GOp &g = ops[before[q]];
                 mul2(g.m, ops[o].m);
                 mul2(g.m, p.m);
+                g.det *= ops[o].det * abs_det(p.m);
                 ops[o].type = G_NONE;
                 open[q] = before[q];
                 before[q] = -1;
@@ -100,6 +118,7 @@ Planner::Planner(const std::vector<qs_prim> &prims, int n_, int dtype_) : n(n_),
             g.type = G_U;
             g.tgt = p.off1;
             memcpy(g.m, p.m, sizeof(g.m));
+            g.det = abs_det(p.m);
             before[q] = (diag_only | x_only) >> q & 1 ? -1 : o;
             open[q] = (int)ops.size();
             diag_only &= ~g.tgt;
@@ -284,7 +303,7 @@ bool Planner::next(uint64_t *qmask, std::vector<int> *pass_ops)
         }
         for (int b = 0; b < n && popc(q) < K; ++b) q |= 1ull << b;
     }
-    std::sort(pass_ops->begin(), pass_ops->end());
+    if (n > K) std::sort(pass_ops->begin(), pass_ops->end());      // more than one round
     *qmask = q;
     return true;
 }
@@ -390,15 +409,18 @@ template bool plan_permute<double>(const Planner &, Permute *);
 namespace {
 
 // p * [[.., ..], [.., ..]] with the pivot p pulled out: the kind (base + 0),
-// r, q and the factor that is left.  Kinds of dense ops keep the matrix.
+// r, q and the factor that is left.  Kinds of dense ops keep the matrix.  What is
+// rounded to T turns the gate by that rounding; p makes up for what it does to
+// the norm: the determinant is that of the gates in the list.
 template <typename T>
-uint8_t classify(const double m[8], T *out, double *p)
+uint8_t classify(const GOp &g, T *out, long double *p)
 {
+    const double *m = g.m;
     *p = 1;
     for (int k = 0; k < 8; ++k) out[k] = (T)m[k];
     if (is_x(m)) return K_X;
     const double tol = 9e-16;            // 4 ulp: products of a few rotations
-    double r, q, piv;
+    double r = 0, q = 0, piv = 1;
     uint8_t kind = K_GEN;
     if (m[1] == 0 && m[3] == 0 && m[5] == 0 && m[7] == 0) {
         if (std::fabs(m[0]) >= std::fabs(m[2])) {
@@ -419,16 +441,18 @@ uint8_t classify(const double m[8], T *out, double *p)
             if (std::fabs(m[5] / piv - 1) < tol) kind = K_IB;
         }
     }
-    if (kind == K_GEN) return kind;
-    out[0] = (T)r;
-    out[1] = (T)q;
-    *p = piv;
-    // r and q rounded to T turn the angle by that rounding; the factor follows,
-    // so that the gate stays unitary to FP64 rounding
-    if (std::fabs(r) == std::fabs(q)) {
-        const double rt = (double)out[0];
-        *p *= std::sqrt((1 + r * r) / (1 + rt * rt));
+    long double det;                     // of what runs
+    if (kind == K_GEN) {
+        piv = 1;
+        det = abs_det(out);
+    } else {
+        out[0] = (T)r;
+        out[1] = (T)q;
+        const long double rq = (long double)out[0] * out[1];
+        det = std::fabs(kind == K_RAP || kind == K_RBP ? 1 - rq : 1 + rq);
     }
+    // sqrt(g.det / det), the gates being unitary up to rounding
+    *p = piv + piv * (g.det - (long double)piv * piv * det) / 2;
     return kind;
 }
 
@@ -527,7 +551,7 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         }
         return count;
     };
-    cd scale(1, 0);
+    cl scale(1, 0);
     double growth = 1;
     int nops = 0, nent = 0;
     const uint32_t low_tile = (1u << LOW) - 1, all_tile = (1u << K) - 1;
@@ -630,11 +654,11 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
         Op<T> &op = S.op[nops];
         memset(&op, 0, sizeof(op));
         if (g.type == G_U) {
-            double p;
+            long double p;
             const int j = reg_bit(g.tgt);
-            const uint8_t kind = classify<T>(g.m, op.m, &p);
+            const uint8_t kind = classify<T>(g, op.m, &p);
             scale *= p;
-            growth /= std::fabs(p);
+            growth /= (double)std::fabs(p);
             // an H right behind the ladder whose hub it mixes: one op
             Op<T> *last = nops > S.st[S.nstages - 1].first ? &S.op[nops - 1] : nullptr;
             if (kind == K_RAM && op.m[0] == 1 && op.m[1] == 1 && last && last->kind == K_LAD + j && !last->cond) {
@@ -687,15 +711,19 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
                 }
             op.kind = op.creg == 0 ? K_LAD0 : (op.creg & (op.creg - 1)) ? K_LADR : K_LAD + low_bit(op.creg);
         }
-        if (g.type == G_DIAG && g.ctrl == 0) scale *= cd(g.m[0], g.m[1]);
+        if (g.type == G_DIAG && g.ctrl == 0) {
+            // m00 and, of what w lost when it was rounded, one half (w has modulus 1):
+            // the other half stays where the qubit is set
+            const cl m00(g.m[0], g.m[1]), m11(g.m[6], g.m[7]), w(op.m[0], op.m[1]);
+            scale = mul(scale, m00 + mul(m11 - mul(m00, w), std::conj(w) * 0.5L));
+        }
         ++nops;
         if (growth > 0x1p8) {                     // the pivots' factors so far, before values grow further
             Op<T> &sc = S.op[nops++];
             memset(&sc, 0, sizeof(sc));
-            const double s = std::abs(scale);
             sc.kind = K_SCALE;
-            sc.m[0] = (T)s;
-            scale /= (double)sc.m[0];
+            sc.m[0] = (T)std::abs(scale);
+            scale /= (long double)sc.m[0];
             growth = 1;
         }
         return true;

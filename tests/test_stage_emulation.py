@@ -15,7 +15,7 @@ import pytest
 
 from oracle.pyoracle import OracleState
 from qpanda_b200 import circuits
-from qpanda_b200.capi import lib
+from qpanda_b200.capi import OP, lib
 from tests.golden.make_golden import every_gate_circuit
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -222,3 +222,47 @@ def test_planning_time_is_linear(emu, n, kind):
         return best / len(gates)
 
     assert per_gate(60000) < 3 * per_gate(2000)
+
+
+def gate_by_gate(init, gates, dtype):
+    """RX, RY, RZ, H and CNOT records on a state of `dtype`, one by one, with the
+    gates' FP64 matrices."""
+    x = init.astype(dtype)
+    for g in gates:
+        op, t, q = int(g["op"]), float(g["theta"]) / 2, [int(k) for k in g["q"]]
+        if op == OP["CNOT"]:
+            i = np.arange(len(x))
+            i = i[(i >> q[0] & 1 == 1) & (i >> q[1] & 1 == 0)]
+            x[i], x[i | 1 << q[1]] = x[i | 1 << q[1]], x[i]
+            continue
+        c, s, h = np.cos(t), np.sin(t), 0.707106781186548
+        m = {OP["RX"]: [[c, -1j * s], [-1j * s, c]], OP["RY"]: [[c, -s], [s, c]],
+             OP["RZ"]: [[c - 1j * s, 0], [0, c + 1j * s]], OP["H"]: [[h, h], [h, -h]]}[op]
+        v = x.reshape(-1, 2, 1 << q[0])
+        a, b = v[:, 0].copy(), v[:, 1].copy()
+        v[:, 0] = dtype(m[0][0]) * a + dtype(m[0][1]) * b
+        v[:, 1] = dtype(m[1][0]) * a + dtype(m[1][1]) * b
+    return x
+
+
+@pytest.mark.parametrize("n,layers", [(9, 8), (12, 20), (10, 60)])
+def test_complex128_is_as_exact_as_gate_by_gate(emu, n, layers):
+    """Against extended precision: the pivots, ratios and phases that a pass rounds
+    must not add up over its gates, in the norm or in the state."""
+    drift, err, plain, passes = [], [], [], 0
+    for seed in range(12):
+        rng = np.random.default_rng(seed)
+        init = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+        init /= np.linalg.norm(init)
+        gates = circuits.random_layers(n, layers, seed)
+        st = init.copy()
+        passes = max(passes, plan(emu, n, gates, C128, st)[0])
+        exact = gate_by_gate(init, gates, np.clongdouble)
+        norm = np.sqrt((np.abs(exact) ** 2).sum())
+        drift.append(float(np.sqrt((np.abs(st.astype(np.clongdouble)) ** 2).sum()) - norm))
+        err.append(float(np.sqrt((np.abs(st - exact) ** 2).sum())))
+        plain.append(float(np.sqrt((np.abs(gate_by_gate(init, gates, np.complex128) - exact) ** 2).sum())))
+    # one rounding of a pass's factor (1.1e-16), and 1e-16 for the phases, whose
+    # rounding is split between the halves of the state
+    assert np.sqrt(np.mean(np.square(drift))) < 1.1e-16 * passes + 1e-16
+    assert np.mean(err) < np.mean(plain)
