@@ -15,6 +15,7 @@
 // Circuits with the same gate pattern (same operations on the same qubits)
 // share one plan structure; only their block matrices are rebuilt.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <functional>
@@ -899,6 +900,7 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
     std::map<std::string, int> proto_of;              // signature -> index in protos
     std::vector<qs_plan *> protos, plans(n_circ, nullptr);
     std::vector<int> proto_id(n_circ), proto_rep;     // proto_rep: a circuit of each structure
+    std::vector<char> finite;                         // every angle of a structure's circuits is
     B->nq.resize(n_circ);
     B->nq_eff.resize(n_circ);
     for (int c = 0; c < n_circ && !r; ++c) {
@@ -911,8 +913,12 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
                 r = qs_fail(QS_ERR_ARG, "qs_batch_create: circuit %d gate %zu uses a qubit >= %d", c, i, n_qubits[c]);
         if (r) break;
         auto ins = proto_of.emplace(signature(B->nq_eff[c], g, cnt), (int)proto_rep.size());
-        if (ins.second) proto_rep.push_back(c);
+        if (ins.second) {
+            proto_rep.push_back(c);
+            finite.push_back(1);
+        }
         proto_id[c] = ins.first->second;
+        for (size_t i = 0; i < cnt; ++i) finite[proto_id[c]] = finite[proto_id[c]] && std::isfinite(g[i].theta);
     }
     // Host work in parallel: the plan of each structure with its pass layouts,
     // then every circuit's block matrices rebound onto its structure's plan.
@@ -944,7 +950,8 @@ extern "C" int qs_batch_create(int n_circ, const int *n_qubits, const qs_gate *g
             const int c = proto_rep[pi];
             const int rr = qs_plan_create_ex(B->nq_eff[c], gates + offsets[c], offsets[c + 1] - offsets[c], &po, &protos[pi]);
             const qs_plan *pp = protos[pi];
-            uint64_t untouched = (1ull << B->nq_eff[c]) - 1;    // qubits still in |0>
+            // qubits still in |0> (zero times infinity would not stay zero)
+            uint64_t untouched = finite[pi] ? (1ull << B->nq_eff[c]) - 1 : 0;
             for (size_t u = 0; !rr && want_tmem && u < pp->passes.size() && tl_ok[pi]; ++u) {
                 // the pass for k_batch_tmem: in place, natural layout
                 const PlanPass &pass = pp->passes[u];

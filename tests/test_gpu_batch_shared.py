@@ -47,3 +47,23 @@ def test_lane_groups_match_oracle(need_gpu, count, width):
     zz = b.zz()
     for k in range(count):
         assert np.abs(zz[k] - refs[2 if k == count - 1 else k % 2]).max() < TOL, k
+
+
+def test_non_finite_angle_reaches_every_amplitude(need_gpu):
+    """Zero times NaN is no zero: tiles that the passes would leave alone take
+    part when a circuit of their structure has an angle that is not finite, as
+    they do in the kernel that leaves none alone.  The highest qubits are idle."""
+    def circuit(n, theta):
+        return n, circuits.make_gates([("RX", (0,), theta)] + [("RY", (q,), 0.3 + q) for q in range(1, 11)])
+
+    sweep = [circuit(14, np.nan), circuit(14, 0.7), circuit(17, np.nan)]
+    states = {}
+    for tmem in (0, 1):
+        b = Batch(sweep, tile_in_tmem=tmem)
+        b.run()
+        assert np.isnan(b.zz()[0]).all() and np.isnan(b.zz()[2]).all()
+        states[tmem] = [b.state(k) for k in range(3)]
+    for k in range(3):
+        assert np.array_equal(np.isnan(states[1][k]), np.isnan(states[0][k])), k
+    assert np.isnan(states[1][0]).all() and np.isnan(states[1][2]).all()
+    assert np.abs(states[1][1] - oracle_zz(*sweep[1])[1]).max() < TOL
