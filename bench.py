@@ -293,6 +293,11 @@ def run_reference(args):
     ws, rank, _ = dist_setup()
     if rank != 0:
         return
+    from oracle.pyoracle import ref_available
+    if not ref_available(True):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref is not built: it is compiled from the "
+                          "reference's own sources, which are not here (make -C oracle ref)"}))
+        return
     n, depth = args.qubits, args.depth
     if args.workload == "circuit20":
         return run_reference_circuit20(args)
