@@ -38,6 +38,7 @@
 #pragma once
 
 #include <cmath>
+#include <complex>
 #include <cstdint>
 #include <cstring>
 #include <vector>
@@ -615,6 +616,10 @@ struct Planner {
     // qubits 0.47 ms, 0.62 with the copies).
     std::vector<Masks> left;
     size_t front = 0;
+    // What the factors of the passes so far lost when they were rounded: the next
+    // pass with a factor owes it.  lost: the same with the pass that plan_pass made
+    // last, which runs when next() is called again.
+    std::complex<long double> owed = 1, lost = 1;
 private:
     int count(uint64_t q) const;
     void take(uint64_t q, std::vector<uint64_t> *wants, std::vector<int> *taken);
@@ -662,6 +667,6 @@ bool plan_permute(const Planner &plan, Permute *P);
 // The stages of a pass (a RunSmall or RunLarge): fills R from pass_ops on the
 // tile of qmask; ops that do not fit R come back in *rest, in order.
 template <typename R, typename T>
-void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_ops, R *out, std::vector<int> *rest);
+void plan_pass(Planner &P, uint64_t qmask, const std::vector<int> &pass_ops, R *out, std::vector<int> *rest);
 
 }  // namespace qs_stg

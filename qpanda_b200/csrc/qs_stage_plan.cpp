@@ -270,6 +270,7 @@ void Planner::take(uint64_t q, std::vector<uint64_t> *wants, std::vector<int> *t
 bool Planner::next(uint64_t *qmask, std::vector<int> *pass_ops)
 {
     pass_ops->clear();
+    owed = lost;
     if (front == left.size()) return false;
     uint64_t q = n <= K ? (1ull << n) - 1 : (1ull << low) - 1;
     std::vector<uint64_t> wants;
@@ -461,7 +462,7 @@ int pair_index(int ja, int jb) { return jb * (jb - 1) / 2 + ja; }
 }  // namespace
 
 template <typename R, typename T>
-void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_ops, R *out, std::vector<int> *rest)
+void plan_pass(Planner &P, uint64_t qmask, const std::vector<int> &pass_ops, R *out, std::vector<int> *rest)
 {
     constexpr int RB = Traits<T>::RB, LB = Traits<T>::LB, LOW = Traits<T>::LOW;
     const int K = popc(qmask), n = P.n, tbits = K - RB;
@@ -793,14 +794,22 @@ void plan_pass(const Planner &P, uint64_t qmask, const std::vector<int> &pass_op
     };
     offsets(S.st[0], reg_in, qubit, S.gin_t, S.gin_r);
     offsets(S.st[S.nstages - 1], reg_at, stored_q, S.gout_t, S.gout_r);
-    S.scale[0] = (T)scale.real();
-    S.scale[1] = (T)scale.imag();
     S.scale_kind = scale.imag() != 0 ? 2 : scale.real() != 1 ? 1 : 0;
+    P.lost = P.owed;
+    if (S.scale_kind) {
+        // with what the passes before lost when their factors were rounded; a real
+        // factor stays one
+        const cl f = S.scale_kind == 2 ? P.owed : cl(P.owed.real(), 0);
+        scale = mul(scale, f);
+        S.scale[0] = (T)scale.real();
+        S.scale[1] = (T)scale.imag();
+        P.lost = P.owed / f * (scale / cl(S.scale[0], S.scale[1]));
+    }
 }
 
-template void plan_pass<RunSmall<float>, float>(const Planner &, uint64_t, const std::vector<int> &, RunSmall<float> *, std::vector<int> *);
-template void plan_pass<RunLarge<float>, float>(const Planner &, uint64_t, const std::vector<int> &, RunLarge<float> *, std::vector<int> *);
-template void plan_pass<RunSmall<double>, double>(const Planner &, uint64_t, const std::vector<int> &, RunSmall<double> *, std::vector<int> *);
-template void plan_pass<RunLarge<double>, double>(const Planner &, uint64_t, const std::vector<int> &, RunLarge<double> *, std::vector<int> *);
+template void plan_pass<RunSmall<float>, float>(Planner &, uint64_t, const std::vector<int> &, RunSmall<float> *, std::vector<int> *);
+template void plan_pass<RunLarge<float>, float>(Planner &, uint64_t, const std::vector<int> &, RunLarge<float> *, std::vector<int> *);
+template void plan_pass<RunSmall<double>, double>(Planner &, uint64_t, const std::vector<int> &, RunSmall<double> *, std::vector<int> *);
+template void plan_pass<RunLarge<double>, double>(Planner &, uint64_t, const std::vector<int> &, RunLarge<double> *, std::vector<int> *);
 
 }  // namespace qs_stg
