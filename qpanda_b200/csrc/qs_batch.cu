@@ -5,10 +5,12 @@
 // width and depth share one launch: every circuit gets its own state buffer
 // (at least 12 qubits: narrower ones are padded with idle qubits that stay in
 // |0>), its own fused plan (tiled passes of up to three 5-qubit tensor-core
-// blocks, qs_plan.cpp), and the kernel's CTAs take whole circuits from a
-// queue, longest first.  A CTA runs all passes of its circuit over all of the
-// circuit's tiles, so passes need no synchronisation between CTAs; states up
-// to a few MB stay in L2 while their CTA works on them.  The first pass starts
+// blocks, qs_plan.cpp), and the kernel's CTAs take circuits from a queue,
+// longest first.  One CTA runs all passes of a circuit over all of the
+// circuit's tiles, so that its passes need no synchronisation between CTAs;
+// states up to a few MB stay in L2 while their CTA works on them.  (The widest
+// circuits of k_batch_tmem are shared among CTAs, part by part, and wait for
+// the parts of the pass before: see there.)  The first pass starts
 // from |0...0> without reading memory; the last pass also accumulates the
 // nearest-neighbour <Z_i Z_{i+1}> expectations of the circuit.
 //

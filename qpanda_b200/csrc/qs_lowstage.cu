@@ -1,5 +1,6 @@
 // qs_lowstage.cu - the per-gate path with runs of gates staged in shared
-// memory and registers.
+// memory and registers.  qs_gates_apply uses it on states of up to 7 qubits,
+// which are one tile; wider ones take staged passes (qs_stage.cu).
 //
 // A gate whose target bits (the pair it mixes, or none for a phase) lie in a
 // set Q of K (= 10) qubits mixes amplitudes inside the tiles of Q: the 2^K

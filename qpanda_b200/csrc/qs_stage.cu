@@ -12,7 +12,7 @@ using namespace qs_stg;
 // Five CTAs per SM in FP32 (48 registers, a few words spilled): an op is a chain
 // of record loads, a jump and multiply-adds, and more warps cover it.  28-qubit
 // depth-16 list on a dense state: three CTAs 37.1 ms, four 32.6, five 27.4, six
-// (40 registers) 31.3; 28-qubit QFT 6.25, 5.63, 5.29, 7.2.  FP64: two CTAs of 512
+// (40 registers) 31.3; 28-qubit QFT 6.25, 5.63, 5.29, 7.2 (5.04 since).  FP64: two CTAs of 512
 // threads, three (40 registers) 15.6 against 13.2 ms (26 qubits, depth 16).
 template <typename T, typename R>
 __global__ void __launch_bounds__(1 << (kMaxTile - Traits<T>::RB), sizeof(T) == 4 ? 5 : 2)
