@@ -269,16 +269,22 @@ int apply_t(qs_state *s, const std::vector<qs_prim> &prims)
             return launch_permute<T>(s, perm);
         }
         if (!P.next(&qmask, &pass)) break;
-        // a pass that would move more than its gates one by one stays with them
+        // a pass that would move more than its gates one by one stays with them,
+        // and so does a lone one (a ladder is as many launches as it has phases)
         double traffic = 0;
-        for (int i : pass) traffic += op_traffic(P, P.ops[(size_t)i]);
+        int launches = 0;
+        for (int i : pass) {
+            const GOp &g = P.ops[(size_t)i];
+            traffic += op_traffic(P, g);
+            launches += g.type == G_DIAG ? g.count : 1;
+        }
         int r = QS_OK;
         const bool zeros = finite && (s->untouched & ~qmask) != 0;
         auto one_by_one = [&]() {
             for (size_t k = 0; !r && k < pass.size(); ++k) r = launch_op(s, P, P.ops[(size_t)pass[k]]);
             return r;
         };
-        if (pass.size() == 1 || (traffic <= 1.0 && s->amp_bytes() >= (64ull << 20))) {
+        if (launches == 1 || (traffic <= 1.0 && s->amp_bytes() >= (64ull << 20))) {
             if (one_by_one()) return r;
             continue;
         }

@@ -2,6 +2,7 @@
 take, one tile, the first states of several tiles, parameter blocks of both
 sizes, and lists that stay on the per-gate kernels."""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -128,3 +129,46 @@ def test_many_phases_on_one_hub_served(need_gpu):
     assert np.abs(srv.fetch_probs(rid) - o.probs()).max() < 1e-5
     srv.release(rid)
     srv.close()
+
+
+def ladder(n):
+    return circuits.make_gates([("CR", (0, q), 0.1 * q) for q in range(1, n)])
+
+
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("n", [8, 11, 12, 13, 16, 23])
+def test_lone_ladder(need_gpu, n, dtype):
+    init, gates = random_state(n, n), ladder(n)
+    with StateVector(n, dtype) as sv:
+        sv.set_state(init.astype(np.complex64) if dtype == "c64" else init)
+        sv.apply(gates)
+        got = sv.get_state()
+    o = OracleState(n)
+    o.set_state(init)
+    o.apply(gates)
+    assert np.abs(got - o.state()).max() < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+def test_lone_ladder_is_one_pass(need_gpu, dtype):
+    """A list that joins into one ladder takes one read and write of the state,
+    not a launch per phase (23 phases of a quarter of the state or more)."""
+    import torch
+
+    n, gates = 24, ladder(24)
+    with StateVector(n, dtype) as sv:
+        def best(f):
+            times = []
+            for _ in range(10):
+                torch.cuda.synchronize()
+                t = time.perf_counter()
+                f()
+                torch.cuda.synchronize()
+                times.append(time.perf_counter() - t)
+            return min(times)
+
+        def one_by_one():
+            for k in range(len(gates)):
+                check(lib().qs_gate_apply(sv.handle, C.c_void_p(gates[k:k + 1].ctypes.data)))
+
+        assert best(lambda: sv.apply(gates)) < 0.6 * best(one_by_one)
