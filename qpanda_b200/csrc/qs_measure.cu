@@ -542,29 +542,45 @@ __global__ void k_shots(const T *__restrict__ a, const double *__restrict__ tree
 // bins of the measured qubits, the outcome tree, then a thread per shot.
 // (256 shots of 9 qubits: four launches and their gaps, 61 us a call, most of
 // it spent around 15 us of kernels.)
-constexpr int kSmallQubits = 11;
+constexpr int kSmallQubits = 11, kSmallLog = 9;                // its threads: 2^kSmallLog
 
 template <typename T>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(1 << kSmallLog)
 k_sample_small(const T *__restrict__ a, int n, int m, const __grid_constant__ ShotParams P,
                const double *__restrict__ u, uint64_t shots, uint64_t *__restrict__ out)
 {
     typedef typename vec2<T>::type V;
-    __shared__ double tree[2 << kSmallQubits];
+    __shared__ double tree[2 << kSmallQubits], part[1 << kSmallLog];
     const V *pa = reinterpret_cast<const V *>(a);
     uint32_t free_bits = (1u << n) - 1;                        // the qubits that are not measured
     for (int k = 0; k < m; ++k) free_bits &= ~(1u << P.qubits[k]);
-    for (uint32_t b = threadIdx.x; b < 1u << m; b += blockDim.x) {
-        uint32_t at = 0;
-        for (int k = 0; k < m; ++k) at |= (b >> k & 1u) << P.qubits[k];
+    // Few bins: 2^share threads to a bin, each with the settings of the free bits
+    // whose lowest `share` are its own (a thread per bin of 1024 amplitudes: 11
+    // qubits complex128, one measured, 138 us a call, where four launches took 43).
+    int share = 0;
+    while (m + share < kSmallLog && m + share < n) ++share;
+    for (uint32_t i = threadIdx.x; i < 1u << (m + share); i += blockDim.x) {
+        uint32_t at = 0, rest = free_bits;
+        for (int k = 0; k < share; ++k, rest &= rest - 1) at |= (i >> k & 1u) ? rest & -rest : 0u;
+        for (int k = 0; k < m; ++k) at |= (i >> (share + k) & 1u) << P.qubits[k];
         double s = 0;
         uint32_t w = 0;
-        do {                                                   // over the settings of the free bits, ascending
+        do {                                                   // over the settings of the rest, ascending
             const V x = pa[at | w];
             s += p2(x.x, x.y);
-            w = (w - free_bits) & free_bits;
+            w = (w - rest) & rest;
         } while (w);
-        tree[(1u << m) + b] = s;
+        if (share) part[i] = s;
+        else tree[(1u << m) + i] = s;
+    }
+    if (share) {
+        const uint32_t i = threadIdx.x, own = i & ((1u << share) - 1);
+        const bool has = i < 1u << (m + share);
+        for (uint32_t step = 1u << (share - 1); step; step >>= 1) {
+            __syncthreads();
+            if (has && own < step) part[i] += part[i + step];
+        }
+        if (has && own == 0) tree[(1u << m) + (i >> share)] = part[i];
     }
     for (int k = m - 1; k >= 0; --k) {
         __syncthreads();
@@ -959,7 +975,7 @@ int sample_t(qs_state *s, const int *qubits, int m, const double *u, size_t shot
     // (many shots are better spread over the device: k_shots)
     if (s->n <= kSmallQubits && shots <= 4096) {
         QS_CUDA_TRY(cudaMemcpyAsync(sc + o_u, u, u_b, cudaMemcpyHostToDevice, s->stream));
-        k_sample_small<T><<<1, 512, 0, s->stream>>>(static_cast<const T *>(s->amp), s->n, m, SP,
+        k_sample_small<T><<<1, 1 << kSmallLog, 0, s->stream>>>(static_cast<const T *>(s->amp), s->n, m, SP,
                                                     reinterpret_cast<const double *>(sc + o_u), shots, res);
         QS_LAUNCH_CHECK("k_sample_small");
         return finish();
