@@ -556,7 +556,7 @@ k_sample_small(const T *__restrict__ a, int n, int m, const __grid_constant__ Sh
     for (int k = 0; k < m; ++k) free_bits &= ~(1u << P.qubits[k]);
     // Few bins: 2^share threads to a bin, each with the settings of the free bits
     // whose lowest `share` are its own (a thread per bin of 1024 amplitudes: 11
-    // qubits complex128, one measured, 138 us a call, where four launches took 43).
+    // qubits complex128, one measured, 138 us a call, so 28).
     int share = 0;
     while (m + share < kSmallLog && m + share < n) ++share;
     for (uint32_t i = threadIdx.x; i < 1u << (m + share); i += blockDim.x) {

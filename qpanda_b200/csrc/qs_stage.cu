@@ -270,7 +270,8 @@ int apply_t(qs_state *s, const std::vector<qs_prim> &prims)
         }
         if (!P.next(&qmask, &pass)) break;
         // a pass that would move more than its gates one by one stays with them,
-        // and so does a lone one (a ladder is as many launches as it has phases)
+        // and so does a lone one (a ladder is as many launches as it has phases: 23
+        // phases of 24 qubits complex128 1063 us so, 96 in a pass)
         double traffic = 0;
         int launches = 0;
         for (int i : pass) {

@@ -216,9 +216,9 @@ def test_planning_time_is_linear(emu, n, kind):
         gates = np.tile(one, max(1, count // len(one)))
         best = 1e9
         for _ in range(3):
-            t = time.perf_counter()
+            t = time.process_time()
             plan(emu, n, gates, C64)
-            best = min(best, time.perf_counter() - t)
+            best = min(best, time.process_time() - t)
         return best / len(gates)
 
     assert per_gate(60000) < 3 * per_gate(2000)
